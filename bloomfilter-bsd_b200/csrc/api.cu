@@ -113,7 +113,16 @@ struct WsHeader {
 };
 static_assert(sizeof(WsHeader) == 128, "header is one 128-byte line");
 
-uint32_t probe_tiles(uint64_t n_phys) { return static_cast<uint32_t>((n_phys + kProbeTile - 1) / kProbeTile); }
+// Status words of the fused plan for up to n_phys keys: those of its largest
+// tiles, or of its smallest where these are used (a bound that never falls as
+// n_phys grows, so a workspace sized for more keys always serves fewer).
+uint64_t probe_tiles(uint64_t n_phys) {
+  return std::max<uint64_t>((n_phys + kProbeTile - 1) / kProbeTile,
+                            std::min<uint64_t>((n_phys + kProbeThreads - 1) / kProbeThreads, kFusedSumTiles));
+}
+static_assert((kFusedOneKey + kProbeThreads - 1) / kProbeThreads <= kFusedSumTiles &&
+                  (kFusedOneRound + kProbeThreads * 4 - 1) / (kProbeThreads * 4) <= kFusedSumTiles,
+              "the status words hold one word per tile of every shape");
 
 // Two-pass layout inside the same workspace: header | status words | bitmask.
 constexpr uint64_t kTwoPassMinKeys = 1ull << 20;
@@ -356,10 +365,14 @@ dtlg_status launch_probe(const dtlg_filter* f, const uint64_t* words, const uint
   const uint64_t n_phys = static_cast<uint64_t>(n) + pre;
   int mode = probe_plan(f, n);
   if (gather && mode == 1) mode = 2;
-  const uint32_t tiles = mode == 1 ? probe_tiles(n_phys) : compact_tiles(n_phys);
+  const FusedShape shape = fused_shape(n_phys);
+  const uint32_t tiles = mode == 1 ? shape.n_tiles : compact_tiles(n_phys);
   const WsLayout lay = ws_layout(n_phys);
   if (ws_bytes < (mode == 3 ? lay.total : lay.total_small)) return DTLG_ERR_WORKSPACE;
-  DTLG_CUDA(cudaMemsetAsync(ws, 0, sizeof(WsHeader) + static_cast<size_t>(tiles) * 8, stream));
+  // a batch of one fused tile takes no ticket and waits for nobody, and the
+  // kernel clears the error word itself
+  const bool one_tile = mode == 1 && tiles == 1;
+  if (!one_tile) DTLG_CUDA(cudaMemsetAsync(ws, 0, sizeof(WsHeader) + static_cast<size_t>(tiles) * 8, stream));
   char* wsb = static_cast<char*>(ws);
   WsHeader* h = static_cast<WsHeader*>(ws);
   ProbeArgs a{};
@@ -383,11 +396,7 @@ dtlg_status launch_probe(const dtlg_filter* f, const uint64_t* words, const uint
     // the fused plan reads Bloom filters that cannot live in L1 without
     // allocating there, as the bitmask plan does (below)
     a.l1na = (f->bk != nullptr && (f->d.m_actual / 8) > kL1NoAllocBytes) ? 1u : 0u;
-    const probe_fn fn = f->pk->probe;
-    const occ_fn occ = f->pk->probe_blocks_per_sm;
-    const int per_sm = std::max(1, occ());
-    const int grid = static_cast<int>(std::min<uint64_t>(tiles, static_cast<uint64_t>(ds->sms) * per_sm));
-    DTLG_CUDA(fn(a, grid, stream));
+    DTLG_CUDA(f->pk->probe(a, shape, ds->sms, stream));
     return DTLG_OK;
   }
   uint32_t* bits = reinterpret_cast<uint32_t*>(wsb + lay.bits_off);

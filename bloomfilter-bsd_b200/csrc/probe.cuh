@@ -4,14 +4,15 @@
 // write i + match_offset (32-bit wrap) for every matching key index i, in
 // ascending order, and return the count.
 //
-// Shape: persistent CTAs of 256 threads pull tiles of 1024*ROUNDS keys from a
-// device counter (so a tile is only ever taken after all earlier tiles were
-// taken by running CTAs: the look-back below cannot deadlock).  Inside a tile,
-// thread t of round r owns the 4 consecutive keys r*1024 + 4t .. +3, loaded as
-// one 16-byte vector; matches are ranked with warp ballots and a CTA scan, and
-// the tile's global offset comes from a decoupled look-back over the per-tile
-// status words.  Every wait is bounded: on timeout the kernel raises the error
-// word and carries on with a zero prefix, so it always terminates.
+// Shape: CTAs of 256 threads pull tiles of 256 to 4096 keys (fused_shape) from
+// a device counter (so a tile is only ever taken after all earlier tiles were
+// taken by running CTAs: the waits below cannot deadlock).  Inside a tile,
+// thread t owns 1 or 4 consecutive keys of each round (4: loaded as one
+// 16-byte vector); matches are ranked with warp ballots and a CTA scan, and
+// the tile's global offset comes from the per-tile status words, summed at
+// once or by a decoupled look-back.  Every wait is bounded: on timeout the
+// kernel raises the error word and carries on with a short prefix, so it
+// always terminates.
 #pragma once
 
 #include <cstdint>
@@ -97,60 +98,121 @@ __device__ __forceinline__ uint32_t look_back(const ProbeArgs& a, uint32_t tile,
   return excl;
 }
 
-// Ops::contains(const ProbeArgs&, uint32_t key) -> bool, branch-free and safe
-// for any key value (block / bucket indexes are always inside the filter).
-template <class Ops, int ROUNDS>
+// Exclusive prefix of this tile as the sum of every earlier tile's aggregate,
+// one status word per thread and step (all threads of the CTA; s_sum: one word
+// per warp).  For grids whose tiles all run at once: their aggregates appear
+// at the same time, so a look-back by 32 would walk the whole list window by
+// window, one L2 round trip each, where this takes one round trip in all.
+// The waits are bounded as in look_back.
+__device__ __forceinline__ uint32_t sum_predecessors(const ProbeArgs& a, uint32_t tile, uint32_t* s_sum) {
+  uint32_t sum = 0, spins = 0;
+  for (uint32_t p = threadIdx.x; p < tile;) {
+    const unsigned long long st = ld_volatile(a.status + p);
+    if (st == 0) {
+      if (++spins > kSpinLimit) {
+        atomicOr(a.err, 1u);
+        break;
+      }
+      __nanosleep(20);
+      continue;
+    }
+    sum += static_cast<uint32_t>(st);
+    p += blockDim.x;
+  }
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if ((threadIdx.x & 31u) == 0) s_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  uint32_t total = 0;
+  for (uint32_t w = 0; w < (blockDim.x >> 5); w++) total += s_sum[w];
+  return total;
+}
+
+// Shape of the fused probe for a batch of n_phys keys: keys per thread and
+// round, rounds per tile, and whether the tile offsets come from
+// sum_predecessors (few tiles) or from look_back.
+struct FusedShape {
+  uint32_t kpt, rounds, tile, n_tiles;
+};
+
+// Up to 1024 keys one tile of four keys per thread, which needs no status
+// word; up to kFusedOneKey keys a thread tests one key (tiles of 256 keys), so
+// that a batch of some ten thousand keys already reaches every SM and no
+// thread waits for four gathers one after the other; up to kFusedOneRound keys
+// four (tiles of 1024); beyond, tiles of 4096 keys, whose fewer status words
+// and tickets count more.  Kernel times against tiles of 4096 keys throughout:
+// 60001 keys (zoned u32 w=16 z=4, 225 KiB) 12.7 -> 9.9 us, 900001 keys (u64 w=8
+// s=8 k=8, 8 MiB) 22.7 -> 13.3 us, 1024 keys 4.2 + 1.5 (the zeroing) -> 3.4 us.
+constexpr uint32_t kMaxRounds = 4;
+constexpr uint64_t kFusedOneKey = 300ull << 10;
+constexpr uint64_t kFusedOneRound = 2ull << 20;
+constexpr uint32_t kFusedSumTiles = 2048;  // offsets by sum_predecessors up to this many tiles
+
+__host__ __device__ inline FusedShape fused_shape(uint64_t n_phys) {
+  FusedShape s{};
+  s.kpt = n_phys > kProbeThreads * 4 && n_phys <= kFusedOneKey ? 1u : 4u;
+  s.rounds = n_phys <= kFusedOneRound ? 1u : kMaxRounds;
+  s.tile = static_cast<uint32_t>(kProbeThreads) * s.kpt * s.rounds;
+  s.n_tiles = static_cast<uint32_t>((n_phys + s.tile - 1) / s.tile);
+  return s;
+}
+
+// Ops::contains(const ProbeArgs&, uint32_t key) -> bool, safe for any key
+// value (block / bucket indexes are always inside the filter).  KPT keys per
+// thread and round, ROUNDS rounds per tile.
+template <class Ops, int KPT, int ROUNDS>
 __global__ void __launch_bounds__(kProbeThreads)
 probe_kernel(const __grid_constant__ ProbeArgs a) {
-  constexpr int kTile = kProbeThreads * 4 * ROUNDS;
-  constexpr int kWarps = kProbeThreads / 32;
+  constexpr uint32_t kRoundKeys = kProbeThreads * KPT;
+  constexpr uint32_t kWarps = kProbeThreads / 32;
   static_assert(ROUNDS * kWarps <= 32, "one warp scans the warp totals");
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_wtot[ROUNDS * kWarps];
   __shared__ uint32_t s_excl;
+  __shared__ uint32_t s_sum[kWarps];
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warp = threadIdx.x >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  const uint4* keys4 = reinterpret_cast<const uint4*>(a.keys_al);
+  const bool by_sum = a.n_tiles <= kFusedSumTiles;
 
   for (;;) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(a.tile_ctr, 1u);
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    if (tile >= a.n_tiles) break;
-    const uint64_t tbase = static_cast<uint64_t>(tile) * kTile;
+    uint32_t tile = 0;
+    if (a.n_tiles > 1) {
+      if (threadIdx.x == 0) s_tile = atomicAdd(a.tile_ctr, 1u);
+      __syncthreads();
+      tile = s_tile;
+      if (tile >= a.n_tiles) break;
+    }
+    const uint64_t tbase = static_cast<uint64_t>(tile) * (kRoundKeys * ROUNDS);
 
     uint32_t flags[ROUNDS];
-    uint32_t lane_excl[ROUNDS];
 #pragma unroll
     for (int r = 0; r < ROUNDS; r++) {
-      const uint64_t p0 = tbase + static_cast<uint64_t>(r) * (kProbeThreads * 4) + threadIdx.x * 4u;
+      const uint64_t p0 = tbase + r * kRoundKeys + threadIdx.x * KPT;
       uint32_t f = 0;
       if (p0 < a.n_phys) {
-        const uint4 kv = __ldcs(keys4 + (p0 >> 2));
-        const uint32_t k[4] = {kv.x, kv.y, kv.z, kv.w};
+        uint32_t k[KPT];
+        if constexpr (KPT == 4) {
+          const uint4 kv = __ldcs(reinterpret_cast<const uint4*>(a.keys_al) + (p0 >> 2));
+          k[0] = kv.x; k[1] = kv.y; k[2] = kv.z; k[3] = kv.w;
+        } else {
+          k[0] = __ldcs(a.keys_al + p0);
+        }
 #pragma unroll
-        for (int q = 0; q < 4; q++) f |= (Ops::contains(a, k[q]) ? 1u : 0u) << q;
+        for (int q = 0; q < KPT; q++) f |= (Ops::contains(a, k[q]) ? 1u : 0u) << q;
         // drop lanes before the first key and past the last one
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
+        for (int q = 0; q < KPT; q++) {
           const uint64_t p = p0 + q;
           if (p < a.pre || p >= a.n_phys) f &= ~(1u << q);
         }
       }
       flags[r] = f;
-      uint32_t tot = 0, ex = 0;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint32_t b = __ballot_sync(0xffffffffu, (f >> q) & 1u);
-        ex += __popc(b & lt_mask);
-        tot += __popc(b);
-      }
-      lane_excl[r] = ex;
+      const uint32_t tot = __reduce_add_sync(0xffffffffu, static_cast<uint32_t>(__popc(f)));
       if (lane == 0) s_wtot[r * kWarps + warp] = tot;
     }
     __syncthreads();
 
+    uint32_t agg = 0;
     if (warp == 0) {
       // exclusive scan of the warp totals in key order (round-major)
       const uint32_t v = lane < ROUNDS * kWarps ? s_wtot[lane] : 0u;
@@ -160,33 +222,41 @@ probe_kernel(const __grid_constant__ ProbeArgs a) {
         const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= static_cast<uint32_t>(d)) incl += t;
       }
-      const uint32_t agg = __shfl_sync(0xffffffffu, incl, 31);
+      agg = __shfl_sync(0xffffffffu, incl, 31);
+      if (lane == 0 && a.n_tiles > 1)
+        st_volatile(a.status + tile, ((tile == 0 || by_sum) ? kFlagPrefix : kFlagAgg) | agg);
       if (lane < ROUNDS * kWarps) s_wtot[lane] = incl - v;
-      uint32_t excl = 0;
-      if (tile == 0) {
-        if (lane == 0) st_volatile(a.status, kFlagPrefix | agg);
-      } else {
-        if (lane == 0) st_volatile(a.status + tile, kFlagAgg | agg);
-        excl = look_back(a, tile, lane);
-        if (lane == 0) st_volatile(a.status + tile, kFlagPrefix | static_cast<uint32_t>(excl + agg));
-      }
-      if (lane == 0) {
-        s_excl = excl;
-        if (tile == a.n_tiles - 1) {
-          const bool failed = *reinterpret_cast<volatile unsigned int*>(a.err) != 0u;
-          *a.count_out = failed ? ~0ull : static_cast<unsigned long long>(excl) + agg;
+      if (!by_sum) {
+        uint32_t excl = 0;
+        if (tile > 0) {
+          excl = look_back(a, tile, lane);
+          if (lane == 0) st_volatile(a.status + tile, kFlagPrefix | static_cast<uint32_t>(excl + agg));
         }
+        if (lane == 0) s_excl = excl;
       }
     }
-    __syncthreads();
+    uint32_t excl;
+    if (by_sum) {
+      excl = sum_predecessors(a, tile, s_sum);  // its barrier also publishes s_wtot
+    } else {
+      __syncthreads();
+      excl = s_excl;
+    }
+    if (threadIdx.x == 0 && tile == a.n_tiles - 1) {
+      if (a.n_tiles == 1) *a.err = 0u;  // the workspace is not zeroed for one tile
+      const bool failed = *reinterpret_cast<volatile unsigned int*>(a.err) != 0u;
+      *a.count_out = failed ? ~0ull : static_cast<unsigned long long>(excl) + agg;
+    }
 
-    const uint32_t excl = s_excl;
 #pragma unroll
     for (int r = 0; r < ROUNDS; r++) {
       uint32_t f = flags[r];
-      if (f == 0) continue;
-      uint32_t pos = excl + s_wtot[r * kWarps + warp] + lane_excl[r];
-      const uint64_t p0 = tbase + static_cast<uint64_t>(r) * (kProbeThreads * 4) + threadIdx.x * 4u;
+      // rank of this thread's matches among the warp's
+      uint32_t rank = 0;
+#pragma unroll
+      for (int q = 0; q < KPT; q++) rank += __popc(__ballot_sync(0xffffffffu, (f >> q) & 1u) & lt_mask);
+      uint32_t pos = excl + s_wtot[r * kWarps + warp] + rank;
+      const uint64_t p0 = tbase + r * kRoundKeys + threadIdx.x * KPT;
       const uint32_t logical0 = static_cast<uint32_t>(p0 - a.pre);
       while (f) {
         const int q = __ffs(f) - 1;
@@ -195,6 +265,7 @@ probe_kernel(const __grid_constant__ ProbeArgs a) {
         pos++;
       }
     }
+    if (a.n_tiles <= gridDim.x) break;  // one tile per CTA
     __syncthreads();
   }
 }

@@ -48,6 +48,7 @@ struct NoAllocHeader {
 static_assert(sizeof(NoAllocHeader) == 128, "one 128-byte line");
 
 constexpr uint64_t kMaxTiles = (static_cast<uint64_t>(DTLG_NOALLOC_MAX_KEYS) + 3 + kProbeTile - 1) / kProbeTile;
+static_assert(kMaxTiles >= kFusedSumTiles, "the smaller tiles of smaller calls fit as well");
 constexpr uint64_t kNoAllocScratchBytes = ((sizeof(NoAllocHeader) + kMaxTiles * 8 + 255) / 256) * 256;
 
 static __device__ __align__(256) unsigned char g_probe_scratch[kNoAllocScratchBytes];
@@ -98,7 +99,8 @@ extern "C" dtlg_status dtlg_batch_contains_noalloc(const dtlg_filter* f, const u
   }
   const uint32_t pre = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(keys) & 15u) >> 2);
   const uint64_t n_phys = static_cast<uint64_t>(key_cnt) + pre;
-  const uint32_t tiles = static_cast<uint32_t>((n_phys + kProbeTile - 1) / kProbeTile);
+  const FusedShape shape = fused_shape(n_phys);
+  const uint32_t tiles = shape.n_tiles;
   const size_t used = sizeof(NoAllocHeader) + static_cast<size_t>(tiles) * 8;
   // the array keeps the previous call's words: clear the counter, the error
   // word and the status words this call will read
@@ -120,9 +122,5 @@ extern "C" dtlg_status dtlg_batch_contains_noalloc(const dtlg_filter* f, const u
   // 256-bit block loads where the words are 32-byte aligned (as every plan of
   // dtlg_batch_contains_async reads them)
   a.vec32 = (reinterpret_cast<uintptr_t>(filter_words) & 31u) == 0 ? 1u : 0u;
-  const probe_fn fn = f->pk->probe;
-  const occ_fn occ = f->pk->probe_blocks_per_sm;
-  const int per_sm = std::max(1, occ());
-  const int grid = static_cast<int>(std::min<uint64_t>(tiles, static_cast<uint64_t>(s->sms) * per_sm));
-  return fn(a, grid, stream) == cudaSuccess ? DTLG_OK : DTLG_ERR_CUDA;
+  return f->pk->probe(a, shape, s->sms, stream) == cudaSuccess ? DTLG_OK : DTLG_ERR_CUDA;
 }

@@ -16,7 +16,7 @@
 
 namespace dtlg {
 
-using probe_fn = cudaError_t (*)(const ProbeArgs&, int grid, cudaStream_t);
+using probe_fn = cudaError_t (*)(const ProbeArgs&, const FusedShape& shape, int sms, cudaStream_t);
 using build_fn = cudaError_t (*)(const BuildArgs&, int grid, cudaStream_t);
 using occ_fn = int (*)();
 using probe_bits_fn = cudaError_t (*)(const ProbeArgs&, uint32_t* bits, int or_into, int grid, cudaStream_t);
@@ -33,7 +33,6 @@ using smem_fn = cudaError_t (*)(const ProbeArgs&, uint32_t* bits, uint32_t words
 // The probe kernels every filter kind provides to the probe plans.
 struct ProbeKernels {
   probe_fn probe;                               // plan 1: fused probe + compaction
-  occ_fn probe_blocks_per_sm;
   probe_bits_fn probe_bits[kBitsVariants];      // plan 2: match bitmask
   occ_fn bits_blocks_per_sm[kBitsVariants];
   pairs_fn probe_pairs[kBitsVariants];          // plan 3: partitioned (null: not offered)
@@ -85,9 +84,8 @@ const BloomKernels* find_bloom(uint32_t word_bytes, uint32_t w, uint32_t s, uint
 const CuckooKernels* find_cuckoo(uint32_t t, uint32_t b);
 int registered_bloom_count();
 
-// Keys per probe tile: 256 threads x 4 keys x kProbeRounds.
-constexpr int kProbeRounds = 4;
-constexpr uint32_t kProbeTile = kProbeThreads * 4 * kProbeRounds;
+// Keys per tile of the fused probe's largest shape: 256 threads x 4 keys x kMaxRounds.
+constexpr uint32_t kProbeTile = kProbeThreads * 4 * kMaxRounds;
 
 #ifdef __CUDACC__
 template <class Ops, int MINB>
@@ -136,14 +134,22 @@ struct PairsLaunch {
 
 template <class Ops>
 struct FusedLaunch {
-  static cudaError_t run(const ProbeArgs& a, int grid, cudaStream_t s) {
-    probe_kernel<Ops, kProbeRounds><<<grid, kProbeThreads, 0, s>>>(a);
+  // a.n_tiles as `shape` has it.  One CTA per tile of the one-round shapes (a
+  // tile waits only for tiles taken before it), the resident CTAs beyond.
+  static cudaError_t run(const ProbeArgs& a, const FusedShape& shape, int sms, cudaStream_t s) {
+    if (shape.kpt == 1) {
+      probe_kernel<Ops, 1, 1><<<a.n_tiles, kProbeThreads, 0, s>>>(a);
+    } else if (shape.rounds == 1) {
+      probe_kernel<Ops, 4, 1><<<a.n_tiles, kProbeThreads, 0, s>>>(a);
+    } else {
+      constexpr auto kernel = probe_kernel<Ops, 4, kMaxRounds>;
+      int occ = 0;
+      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kProbeThreads, 0);
+      if (e != cudaSuccess) return e;
+      const uint32_t resident = static_cast<uint32_t>(sms) * static_cast<uint32_t>(std::max(1, occ));
+      kernel<<<std::min(a.n_tiles, resident), kProbeThreads, 0, s>>>(a);
+    }
     return cudaGetLastError();
-  }
-  static int occupancy() {
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, probe_kernel<Ops, kProbeRounds>, kProbeThreads, 0);
-    return n;
   }
 };
 
@@ -194,7 +200,7 @@ ProbeKernels probe_entry() {
   using B4 = BitsLaunch<Ops, 4>;
   using P8 = PairsLaunch<Ops, 8>;
   using P4 = PairsLaunch<Ops, 4>;
-  ProbeKernels k{&F::run, &F::occupancy, {&B8::run, &B4::run}, {&B8::occupancy, &B4::occupancy},
+  ProbeKernels k{&F::run, {&B8::run, &B4::run}, {&B8::occupancy, &B4::occupancy},
                  {nullptr, nullptr}, {nullptr, nullptr}, nullptr, {&B8::local_bytes, &B4::local_bytes},
                  {nullptr, nullptr}};
   if constexpr (Smem) k.probe_smem = &SmemLaunch<Ops>::run;

@@ -1,0 +1,42 @@
+"""The fused probe (plan 1) at the edges of its tile shapes: match lists equal
+the oracle's where a batch goes from one tile to several, from one key per
+thread to four, and from tiles of one round to tiles of four."""
+import numpy as np
+import pytest
+
+import dtlg as F
+import oracle as O
+from dtlg import keygen
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+EDGES = [1024, 256 * 5, 300 << 10, 2 << 20]
+N_BUILD = 40000
+
+
+@pytest.fixture(scope="module", params=[(8, 8, 8, 1, 8), (4, 1, 1, 1, 4)], ids=["sectorized", "register"])
+def case(request):
+    wb, w, s, z, k = request.param
+    m = N_BUILD * 12
+    ob, f = O.Bloom(wb, w, s, z, k, m), F.construct(F.blocked_bloomfilter_config(k, wb, w, s, 0, z), m)
+    ref = ob.alloc()
+    ob.insert(ref, keygen.build_keys(N_BUILD, 8))
+    words = torch.zeros(f.alloc_words(), dtype=torch.int64)
+    words[:len(ref)] = torch.from_numpy(ref.view(np.int64))
+    pk, _ = keygen.probe_keys(N_BUILD, max(EDGES) + 4, 0.3, 8)
+    f.set_probe_options(1, -1)
+    return f, words.cuda(), torch.from_numpy(pk.view(np.int32)).cuda(), ob.batch_contains(ref, pk, 0)
+
+
+@pytest.mark.parametrize("edge", EDGES)
+def test_fused_probe_at_shape_edges(case, edge):
+    f, words, keys, exp = case
+    for n in (edge - 1, edge, edge + 1):
+        for pad in (0, 3):
+            want = exp[(exp >= pad) & (exp < pad + n)] - np.uint32(pad) + np.uint32(7)
+            out = torch.full((n + 1,), -1, dtype=torch.int32, device="cuda")
+            got = f.batch_contains(words, keys[pad:pad + n], n, out, 7)
+            assert got == len(want), (n, pad)
+            assert np.array_equal(out[:got].cpu().numpy().view(np.uint32), want), (n, pad)
+            assert bool((out[got:] == -1).all()), (n, pad)
