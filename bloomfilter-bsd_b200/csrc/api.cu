@@ -485,6 +485,88 @@ int block_build_plan(const dtlg_filter* f, uint64_t n) {
   return (f->bk != nullptr && n >= kTwoPassMinKeys && bytes > (80ull << 20)) ? 2 : 1;
 }
 
+// The range-by-range build (build_ranges.cuh) of a blocked Bloom filter from
+// n_phys keys: fills in its ranges and bucket capacity, false where another
+// plan is taken.  It reads and writes every word once and handles 110 to 250
+// Gkeys/s whatever the filter's size, where the one-kernel build does 75 to
+// 180 in L2, by the sectors and words a key touches, and the coarse partition
+// 65 to 90 beyond.  Per-build us, other plan -> range by range:
+//   beyond 80 MiB, one key per 40 bytes or more: u64 w=8 s=8 k=8 2^26 keys /
+//   128 MiB 1002 -> 508, 2^22 / 181 MiB 130 -> 107; u32 w=1 k=4 610 -> 390, 121
+//   -> 114 (at 64 bytes per key 142 -> 144, and u32 w=16 s=8 133 -> 151);
+//   in L2, blocks of 64 bytes whose words all take bits (two sectors per key)
+//   or are picked one by one, one key per 8 bytes or more: u64 w=8 s=8 2^22 /
+//   8 MiB 58 -> 45, 2^24 / 64 MiB 229 -> 164 (2^22 / 64 MiB 58 -> 65); u32
+//   w=16 z=2 2^23 / 16 MiB 86 -> 63; u64 w=8 s=2 2^22 / 8 MiB 81 -> 44;
+//   other layouts in L2 only for very many keys: 2^26 / 64 MiB u32 w=1 390 ->
+//   340, u64 w=4 s=4 634 -> 577, u64 w=8 z=4 633 -> 602, but 2^24 / 32 MiB 93
+//   -> 105, 150 -> 168, 150 -> 175.
+bool range_build(const dtlg_filter* f, uint64_t n_phys, RangeArgs* a, uint32_t* range_bytes) {
+  if (!f->bk || f->build_mode != 0 || n_phys < (1ull << 22) || n_phys > 0x70000000ull) return false;
+  const uint64_t bytes = (f->d.m_actual + 7) / 8;
+  const uint64_t block_bytes = static_cast<uint64_t>(f->d.w) * f->d.word_bytes;
+  const bool wide = block_bytes >= 64 && (f->d.kind == Kind::kBloom || f->d.word_bytes == 4);
+  if (bytes > (80ull << 20) ? bytes > 40 * n_phys : !(wide ? bytes <= 8 * n_phys : n_phys >= (48ull << 20)))
+    return false;
+  // the largest ranges that still make 512 of them (a few per SM): longer runs
+  // for the scatter (2^27 keys over 2048 / 4096 ranges: 496 / 668 us)
+  uint32_t rb = kBuildRangeBytes;
+  while (rb > (8u << 10) && bytes / rb < 512) rb /= 2;
+  a->range_log2 = 0;
+  while ((block_bytes << a->range_log2) < rb) a->range_log2++;
+  const uint64_t ranges = (f->d.addr.block_cnt + (1ull << a->range_log2) - 1) >> a->range_log2;
+  if (ranges < 2 || ranges > kBuildMaxRanges) return false;
+  a->n_ranges = static_cast<uint32_t>(ranges);
+  a->range_shift = 32 - clog2(f->d.addr.block_cnt) + a->range_log2;  // POW2 only
+  const uint64_t share = (n_phys << a->range_log2) / f->d.addr.block_cnt + 1;
+  a->cap = static_cast<uint32_t>((share + share / 32 + 512 + 3) & ~3ull);
+  *range_bytes = rb;
+  return true;
+}
+
+// Enqueues the range-by-range build; cudaErrorMemoryAllocation when there is
+// no room for the buckets (4.1 bytes per key), with nothing enqueued.
+cudaError_t launch_range_build(const dtlg_filter* f, uint64_t* words, const uint32_t* keys_al, uint64_t n_phys,
+                               uint32_t pre, RangeArgs ra, uint32_t range_bytes, const DeviceState& ds,
+                               cudaStream_t stream) {
+  const size_t bucket_bytes = round256(static_cast<uint64_t>(ra.n_ranges) * ra.cap * 4);
+  char* ws = nullptr;
+  if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), bucket_bytes + ra.n_ranges * 4, ds.pool, stream) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return cudaErrorMemoryAllocation;
+  }
+  ra.keys_al = keys_al;
+  ra.n_phys = n_phys;
+  ra.pre = pre;
+  ra.addr = f->d.addr;
+  ra.buckets = reinterpret_cast<uint32_t*>(ws);
+  ra.fill = reinterpret_cast<unsigned int*>(ws + bucket_bytes);
+  ra.filter = words;
+  // a range of the largest size has an SM to itself: while it is built, the
+  // one that the SM takes next comes into L2 (2^22 keys / 256 MiB 154 -> 132
+  // us; smaller ranges share the SM, and the hint only cost: 161 -> 181)
+  ra.prefetch = range_bytes == kBuildRangeBytes ? static_cast<uint32_t>(ds.sms) : 0u;
+  ra.word_bytes = f->d.word_bytes;
+  ra.w = f->d.w;
+  ra.sched = make_schedule(f->d.word_bytes * 8, f->d.w, f->d.s, f->d.z, f->d.k, true);
+  ra.n_tiles = static_cast<uint32_t>((n_phys + kScatterTile - 1) / kScatterTile);
+  const auto scatter = ra.addr.magic_mode ? key_scatter_kernel<true> : key_scatter_kernel<false>;
+  const size_t smem = kScatterTile * 4 + ra.n_ranges * 8;
+  int occ = 0;
+  cudaError_t e = cudaMemsetAsync(ra.fill, 0, ra.n_ranges * 4, stream);
+  if (e == cudaSuccess) e = allow_dynamic_smem(scatter, smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, scatter, kScatterThreads, smem);
+  if (e == cudaSuccess) {
+    const uint32_t grid = std::min<uint32_t>(ra.n_tiles, static_cast<uint32_t>(ds.sms) * std::max(1, occ));
+    scatter<<<grid, kScatterThreads, smem, stream>>>(ra);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = f->bk->build_ranges(ra, range_bytes, stream);
+  cudaFreeAsync(ws, stream);
+  return e;
+}
+
 int grid_for(uint64_t items, int sms) {
   return static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>((items + 255) / 256, static_cast<uint64_t>(sms) * 8)));
 }
@@ -719,6 +801,17 @@ dtlg_status dtlg_batch_insert(const dtlg_filter* f, uint64_t* words, const uint3
     return DTLG_OK;
   }
   const uint64_t n_phys = static_cast<uint64_t>(n) + pre;
+  RangeArgs ra{};
+  uint32_t range_bytes = 0;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  if (range_build(f, n_phys, &ra, &range_bytes) &&
+      cudaStreamIsCapturing(stream, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {
+    const cudaError_t e = launch_range_build(f, words, keys - pre, n_phys, pre, ra, range_bytes, *ds, stream);
+    if (e != cudaErrorMemoryAllocation) {
+      DTLG_CUDA(e);
+      return DTLG_OK;
+    }
+  }
   if (block_build_plan(f, n) == 2) {
     // keys grouped by L2-sized block range first (the probe's partition), then
     // inserted range by range: the atomic ORs hit lines that sit in L2

@@ -8,6 +8,7 @@
 
 #include "bcf.cuh"
 #include "bloom.cuh"
+#include "build_ranges.cuh"
 #include "classic.cuh"
 #include "cuckoo.cuh"
 #include "probe.cuh"
@@ -48,6 +49,8 @@ struct BloomKernels {
   build_fn build;
   // build from range-grouped (key, position) pairs
   cudaError_t (*build_pairs)(const PartArgs& part, void* filter, const Addr& addr, int grid, cudaStream_t);
+  // build from range buckets, one CTA per range of range_bytes
+  cudaError_t (*build_ranges)(const RangeArgs& a, uint32_t range_bytes, cudaStream_t);
 };
 
 struct CuckooKernels {
@@ -165,6 +168,28 @@ struct BloomLaunch {
   }
 };
 
+// Raises the kernel's dynamic shared-memory limit to `bytes` on the current
+// device (a few hundred ns; the limit belongs to the device's context; up to
+// 40 KiB fits the default limit of 48 beside the static shared memory).
+template <class K>
+cudaError_t allow_dynamic_smem(K kernel, size_t bytes) {
+  return bytes <= (40u << 10) ? cudaSuccess
+                              : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     static_cast<int>(bytes));
+}
+
+template <class Cfg>
+struct BloomRangesLaunch {
+  static cudaError_t run(const RangeArgs& a, uint32_t range_bytes, cudaStream_t s) {
+    // a range of the largest size has an SM to itself, smaller ones share it
+    const int threads = range_bytes == kBuildRangeBytes ? 1024 : 512;
+    cudaError_t e = allow_dynamic_smem(bloom_build_ranges_kernel<Cfg>, range_bytes);
+    if (e != cudaSuccess) return e;
+    bloom_build_ranges_kernel<Cfg><<<a.n_ranges, threads, range_bytes, s>>>(a);
+    return cudaGetLastError();
+  }
+};
+
 template <class Ops>
 struct SmemLaunch {
   static cudaError_t run(const ProbeArgs& a, uint32_t* bits, uint32_t words32, uint64_t chunks, int sms,
@@ -219,7 +244,7 @@ template <typename Word, int W, int S, int Z, int K>
 BloomKernels bloom_entry() {
   using C = BloomCfg<Word, W, S, Z, K>;
   return BloomKernels{static_cast<uint32_t>(sizeof(Word)), W, S, Z, K, probe_entry<BloomOps<C>, true, true>(),
-                      &BloomLaunch<C>::build, &BloomLaunch<C>::build_pairs};
+                      &BloomLaunch<C>::build, &BloomLaunch<C>::build_pairs, &BloomRangesLaunch<C>::run};
 }
 
 template <int T, int B>
