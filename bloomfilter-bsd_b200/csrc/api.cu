@@ -579,16 +579,19 @@ dtlg_status cuckoo_insert(const dtlg_filter* f, uint64_t* words, const uint32_t*
   if (failed_out) *failed_out = 0;
   if (n == 0) return DTLG_OK;
   const FilterDesc& d = f->d;
-  const uint64_t slots_n = (static_cast<uint64_t>(d.addr.block_cnt) + 1) * d.b;
+  const bool packed = f->ck->word_bucket;
+  const uint64_t slots_n = packed ? 0 : (static_cast<uint64_t>(d.addr.block_cnt) + 1) * d.b;
   uint32_t* slots = nullptr;
   unsigned long long* failed = nullptr;
   const uint64_t slot_bytes = (slots_n * 4 + 255) & ~255ull;
   DTLG_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&slots), slot_bytes + 256, ds->pool, stream));
   failed = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(slots) + slot_bytes);
   DTLG_CUDA(cudaMemsetAsync(failed, 0, 8, stream));
-  DTLG_CUDA(cudaMemsetAsync(slots + static_cast<uint64_t>(d.addr.block_cnt) * d.b, 0, d.b * 4, stream));
   uint32_t* table = reinterpret_cast<uint32_t*>(words);
-  f->ck->unpack(table, slots, d.addr.block_cnt, grid_for(slots_n, ds->sms), stream);
+  if (!packed) {
+    DTLG_CUDA(cudaMemsetAsync(slots + static_cast<uint64_t>(d.addr.block_cnt) * d.b, 0, d.b * 4, stream));
+    f->ck->unpack(table, slots, d.addr.block_cnt, grid_for(slots_n, ds->sms), stream);
+  }
   const uint32_t pre = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(keys) & 15u) >> 2);
   CuckooBuildArgs a{};
   a.table = table;
@@ -602,8 +605,10 @@ dtlg_status cuckoo_insert(const dtlg_filter* f, uint64_t* words, const uint32_t*
   a.failed = failed;
   static std::atomic<uint64_t> seed_ctr{0x243F6A8885A308D3ull};
   a.seed = seed_ctr.fetch_add(0x9E3779B97F4A7C15ull);
-  f->ck->insert(a, grid_for(a.n_phys, ds->sms), stream);
-  f->ck->pack(table, slots, d.addr.block_cnt, d.word_cnt, grid_for(d.word_cnt, ds->sms), stream);
+  // one key per thread and no more: a thread held up by a long chain of kicks
+  // keeps no other keys waiting
+  f->ck->insert(a, static_cast<int>(std::min<uint64_t>((a.n_phys + 255) / 256, 1u << 22)), stream);
+  if (!packed) f->ck->pack(table, slots, d.addr.block_cnt, d.word_cnt, grid_for(d.word_cnt, ds->sms), stream);
   unsigned long long lost = 0;
   DTLG_CUDA(cudaMemcpyAsync(&lost, failed, 8, cudaMemcpyDeviceToHost, stream));
   DTLG_CUDA(cudaFreeAsync(slots, stream));

@@ -12,13 +12,16 @@
 // Build: the reference inserts one key at a time and picks kick slots with a
 // thread-local mt19937 seeded from std::random_device (cuckoofilter_table.hpp:
 // 197, thread.hpp:72-78), so no two of its builds agree.  The GPU build runs
-// the same bounded-kick partial-key algorithm for all keys at once on an
-// unpacked copy of the table (one 32-bit slot per tag, atomicCAS to claim an
-// empty slot, atomicExch to kick), then packs it back into the reference
-// layout.  Checked by invariants (no false negatives, occupancy) and FPR.
+// the same bounded-kick partial-key algorithm for all keys at once, each key
+// starting in the emptier of its two buckets.  Buckets that are a whole 16-,
+// 32- or 64-bit word are updated in the table itself, one compare-and-swap per
+// step; the others on an unpacked copy (one 32-bit slot per tag), which is
+// packed back afterwards.  Checked by invariants (no false negatives,
+// occupancy) and FPR.
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include "common.cuh"
 #include "probe.cuh"
@@ -32,12 +35,14 @@ template <int T, int B>
 struct CuckooCfg {
   static constexpr int kT = T, kB = B;
   static constexpr int kBytesPerBucket = (T * B + 7) / 8;
+  // the bucket is one 16-, 32- or 64-bit word of the table
+  static constexpr bool kWordBucket = kBytesPerBucket == 2 || kBytesPerBucket == 4 || kBytesPerBucket == 8;
   static constexpr uint32_t kTagMask = T == 32 ? 0xffffffffu : ((1u << T) - 1u);
 };
 
 struct CuckooBuildArgs {
   uint32_t* table;          // packed table (32-bit words) + victim record
-  uint32_t* slots;          // unpacked: (bucket_cnt + 1) * B slots
+  uint32_t* slots;          // unpacked: (bucket_cnt + 1) * B slots (buckets that are no word)
   const uint32_t* keys_al;
   uint64_t n_phys;
   uint32_t pre;
@@ -146,49 +151,208 @@ __device__ __forceinline__ uint32_t kick_rand(uint64_t& s) {  // xorshift64* (Vi
   return static_cast<uint32_t>((s * 2685821657736338717ull) >> 32);
 }
 
-// cuckoofilter_logic.hpp:292-322, all keys in parallel on the slot array.
+__device__ __forceinline__ unsigned short bucket_cas(unsigned short* p, unsigned short c, unsigned short v) {
+  return atomicCAS(p, c, v);
+}
+__device__ __forceinline__ unsigned int bucket_cas(unsigned int* p, unsigned int c, unsigned int v) {
+  return atomicCAS(p, c, v);
+}
+__device__ __forceinline__ unsigned long long bucket_cas(unsigned long long* p, unsigned long long c,
+                                                         unsigned long long v) {
+  return atomicCAS(p, c, v);
+}
+
+// Buckets that are one word of the packed table.  A bucket's value is what a
+// load or a lost compare-and-swap last saw.
+template <class Cfg>
+struct WordBuckets {
+  static constexpr int kT = Cfg::kT, kB = Cfg::kB;
+  using Word = typename std::conditional<Cfg::kBytesPerBucket == 8, unsigned long long,
+                                         typename std::conditional<Cfg::kBytesPerBucket == 4, unsigned int,
+                                                                   unsigned short>::type>::type;
+  using Value = Word;
+  __device__ __forceinline__ static Word* at(const CuckooBuildArgs& a, uint32_t i) {
+    return reinterpret_cast<Word*>(a.table) + i;
+  }
+  __device__ __forceinline__ static Value load(const CuckooBuildArgs& a, uint32_t i) { return __ldcg(at(a, i)); }
+  __device__ __forceinline__ static uint32_t tag_of(Value v, int j) {
+    return static_cast<uint32_t>(v >> (kT * j)) & Cfg::kTagMask;
+  }
+  __device__ __forceinline__ static uint32_t free_slots(const Value& v) {
+    uint32_t n = 0;
+#pragma unroll
+    for (int j = 0; j < kB; j++) n += tag_of(v, j) == 0u;
+    return n;
+  }
+  // The shift of the first empty slot, -1 when the bucket is full.
+  __device__ __forceinline__ static int empty_slot(const Value& v) {
+    int sh = -1;
+#pragma unroll
+    for (int j = kB - 1; j >= 0; j--)
+      if (tag_of(v, j) == 0u) sh = kT * j;
+    return sh;
+  }
+  // The tag into an empty slot of bucket i, false when it is full (or after
+  // kRaces lost races: the key then goes on to its other bucket).
+  static constexpr int kRaces = 64;
+  __device__ __forceinline__ static bool insert(const CuckooBuildArgs& a, uint32_t i, Value& v, uint32_t tag) {
+    for (int n = 0; n < kRaces; n++) {
+      const int sh = empty_slot(v);
+      if (sh < 0) return false;
+      const Word seen = bucket_cas(at(a, i), v, static_cast<Word>(v | static_cast<Word>(tag) << sh));
+      if (seen == v) return true;
+      v = seen;
+    }
+    return false;
+  }
+  // Swaps the tag with the one in slot r and returns that; 0: it went into an
+  // empty slot.  Equal tags need no swap: thousands of copies of one key, more
+  // than its buckets can hold, must not fight over the two words.
+  __device__ __forceinline__ static uint32_t kick(const CuckooBuildArgs& a, uint32_t i, Value& v, uint32_t tag,
+                                                  uint32_t r) {
+    for (int n = 0; n < kRaces; n++) {
+      if (insert(a, i, v, tag)) return 0u;
+      const uint32_t old = tag_of(v, static_cast<int>(r));
+      if (old == tag || old == 0u) break;
+      const Word seen =
+          bucket_cas(at(a, i), v, static_cast<Word>(v ^ static_cast<Word>(old ^ tag) << (kT * r)));
+      if (seen == v) return old;
+      v = seen;
+    }
+    return tag;
+  }
+};
+
+// Buckets of one 32-bit slot per tag in the unpacked copy.
+template <class Cfg>
+struct SlotBuckets {
+  static constexpr int kB = Cfg::kB;
+  struct Value {
+    uint32_t tag[kB];
+  };
+  __device__ __forceinline__ static uint32_t* at(const CuckooBuildArgs& a, uint32_t i) {
+    return a.slots + static_cast<uint64_t>(i) * kB;
+  }
+  __device__ __forceinline__ static Value load(const CuckooBuildArgs& a, uint32_t i) {
+    Value v;
+    if constexpr (kB == 4) {
+      const uint4 x = __ldcg(reinterpret_cast<const uint4*>(at(a, i)));
+      v.tag[0] = x.x; v.tag[1] = x.y; v.tag[2] = x.z; v.tag[3] = x.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < kB; j++) v.tag[j] = __ldcg(at(a, i) + j);
+    }
+    return v;
+  }
+  __device__ __forceinline__ static uint32_t tag_of(const Value& v, int j) { return v.tag[j]; }
+  __device__ __forceinline__ static uint32_t free_slots(const Value& v) {
+    uint32_t n = 0;
+#pragma unroll
+    for (int j = 0; j < kB; j++) n += v.tag[j] == 0u;
+    return n;
+  }
+  __device__ __forceinline__ static bool insert(const CuckooBuildArgs& a, uint32_t i, Value& v, uint32_t tag) {
+    bool done = false;
+#pragma unroll
+    for (int j = 0; j < kB; j++) {
+      if (!done && v.tag[j] == 0u) {
+        v.tag[j] = atomicCAS(at(a, i) + j, 0u, tag);
+        done = v.tag[j] == 0u;
+      }
+    }
+    return done;
+  }
+  __device__ __forceinline__ static uint32_t kick(const CuckooBuildArgs& a, uint32_t i, Value&, uint32_t tag,
+                                                  uint32_t r) {
+    return atomicExch(at(a, i) + r, tag);
+  }
+};
+
+// cuckoofilter_logic.hpp:292-322 for one key.  The reference tries bucket 1,
+// then bucket 2; here both are loaded at once and the emptier one is tried
+// first, which keeps the buckets level.
+template <class Cfg, class S>
+__device__ __forceinline__ void cuckoo_insert_key(const CuckooBuildArgs& a, uint32_t key) {
+  constexpr int kB = Cfg::kB;
+  const uint32_t c = a.addr.block_cnt;  // bucket c lies past the table: never written here
+  uint32_t cur, tag;
+  CuckooOps<Cfg>::index_tag(key, a.addr, cur, tag);
+  uint32_t other = cuckoo_alt(cur, tag, a.addr);
+  typename S::Value v = S::load(a, cur), w = S::load(a, other < c ? other : cur);
+  if (other < c && S::free_slots(w) > S::free_slots(v)) {
+    const uint32_t i = cur;
+    cur = other;
+    other = i;
+    const typename S::Value x = v;
+    v = w;
+    w = x;
+  }
+  bool done = S::insert(a, cur, v, tag);
+  if (!done) {
+    cur = other;
+    if (cur < c) done = S::insert(a, cur, w, tag);
+    v = w;
+  }
+  uint64_t rng = a.seed ^ (0x9E3779B97F4A7C15ull * (static_cast<uint64_t>(key) + 1));
+  // `cur` was full when last seen (as v).  A kick takes a slot whose tag has
+  // room in its other bucket, if there is one (all of them are looked at at
+  // once), else a random one: the kernel ends with its longest chain of kicks.
+  for (uint32_t count = 0; count < kMaxKicks && !done; count++) {
+    if (cur < c) {
+      uint32_t to[kB];
+      typename S::Value x[kB];
+#pragma unroll
+      for (int j = 0; j < kB; j++) {
+        to[j] = cuckoo_alt(cur, S::tag_of(v, j), a.addr);
+        x[j] = S::load(a, to[j] < c ? to[j] : cur);
+      }
+      uint32_t r = kick_rand(rng) % kB;
+      const uint32_t at = r;
+#pragma unroll
+      for (int j = 0; j < kB; j++) {
+        // not always the first with room: keys that kick from one bucket at
+        // the same time then pick different slots
+        if (to[j] < c && S::free_slots(x[j]) != 0u && (r == at || static_cast<uint32_t>(j) < at)) r = j;
+      }
+      const uint32_t old = S::kick(a, cur, v, tag, r);
+      if (old == 0u) {
+        done = true;
+        break;
+      }
+      tag = old;
+    }
+    cur = cuckoo_alt(cur, tag, a.addr);
+    if (cur < c) {
+      v = S::load(a, cur);
+      done = S::insert(a, cur, v, tag);
+    }
+  }
+  if (!done) {
+    // victim cache (cuckoofilter_logic.hpp:318-320); when it is taken the
+    // tag in hand is lost, the reference's `insert == false`.
+    uint32_t* vr = a.table + a.victim_word;
+    if (atomicCAS(vr + 2, 0u, 1u) == 0u) {
+      vr[0] = cur;
+      vr[1] = tag;
+    } else {
+      atomicAdd(a.failed, 1ull);
+    }
+  }
+}
+
+// All keys in parallel, one per thread.  Bound by the chains of dependent L2
+// round trips (key, buckets, compare-and-swap, then the kicks of the few keys
+// that find both buckets full) and by the longest of them; four keys per
+// thread with their loads and first swaps in flight together was slower (129
+// against 103 us: the buckets are chosen on older counts, so more keys kick).
+// t=16 b=4, 3 000 001 keys at load 0.9: 199 us with unpack, pack and random
+// kicks, 103 us so; 2^26 keys at load 0.95 7.4 -> 2.8 ms.
 template <class Cfg>
 __global__ void __launch_bounds__(256) cuckoo_insert_kernel(const __grid_constant__ CuckooBuildArgs a) {
-  constexpr int kB = Cfg::kB;
-  const uint32_t c = a.addr.block_cnt;
+  using S = typename std::conditional<Cfg::kWordBucket, WordBuckets<Cfg>, SlotBuckets<Cfg>>::type;
   for (uint64_t p = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; p < a.n_phys;
        p += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-    if (p < a.pre) continue;
-    const uint32_t key = __ldg(a.keys_al + p);
-    uint32_t cur, tag;
-    CuckooOps<Cfg>::index_tag(key, a.addr, cur, tag);
-    uint64_t rng = a.seed ^ (0x9E3779B97F4A7C15ull * (p + 1));
-    bool done = false;
-    for (uint32_t count = 0; count < kMaxKicks && !done; count++) {
-      if (cur < c) {  // bucket c lies past the table: never written here
-        uint32_t* b = a.slots + static_cast<uint64_t>(cur) * kB;
-#pragma unroll
-        for (int j = 0; j < kB; j++) {
-          if (!done && b[j] == 0u && atomicCAS(b + j, 0u, tag) == 0u) done = true;
-        }
-        if (!done && count > 0) {
-          const uint32_t r = kick_rand(rng) % kB;
-          const uint32_t old = atomicExch(b + r, tag);
-          if (old == 0u) {
-            done = true;
-          } else {
-            tag = old;
-          }
-        }
-      }
-      if (!done) cur = cuckoo_alt(cur, tag, a.addr);
-    }
-    if (!done) {
-      // victim cache (cuckoofilter_logic.hpp:318-320); when it is taken the
-      // tag in hand is lost, the reference's `insert == false`.
-      uint32_t* v = a.table + a.victim_word;
-      if (atomicCAS(v + 2, 0u, 1u) == 0u) {
-        v[0] = cur;
-        v[1] = tag;
-      } else {
-        atomicAdd(a.failed, 1ull);
-      }
-    }
+    if (p >= a.pre) cuckoo_insert_key<Cfg, S>(a, __ldg(a.keys_al + p));
   }
 }
 

@@ -55,6 +55,7 @@ struct BloomKernels {
 
 struct CuckooKernels {
   uint32_t t, b;
+  bool word_bucket;  // insert works on the packed table: no unpack, no pack
   ProbeKernels pk;
   void (*unpack)(const uint32_t* table, uint32_t* slots, uint32_t buckets, int grid, cudaStream_t);
   void (*insert)(const CuckooBuildArgs&, int grid, cudaStream_t);
@@ -270,7 +271,7 @@ struct CuckooLaunch {
 template <int T, int B>
 CuckooKernels cuckoo_entry() {
   using L = CuckooLaunch<T, B>;
-  return CuckooKernels{T, B, probe_entry<CuckooOps<CuckooCfg<T, B>>, false>(), &L::unpack, &L::insert, &L::pack,
+  return CuckooKernels{T, B, CuckooCfg<T, B>::kWordBucket, probe_entry<CuckooOps<CuckooCfg<T, B>>, false>(), &L::unpack, &L::insert, &L::pack,
                        &L::count};
 }
 
