@@ -128,11 +128,15 @@ static_assert((kFusedOneKey + kProbeThreads - 1) / kProbeThreads <= kFusedSumTil
 constexpr uint64_t kTwoPassMinKeys = 1ull << 20;
 uint64_t bits_words(uint64_t n_phys) { return (n_phys + 31) / 32; }
 uint32_t compact_tiles(uint64_t n_phys) {
-  return static_cast<uint32_t>((bits_words(n_phys) + kCompactTileWords - 1) / kCompactTileWords);
+  const uint64_t words = bits_words(n_phys), tile = kCompactThreads * compact_rows(words);
+  return static_cast<uint32_t>((words + tile - 1) / tile);
 }
 size_t status_bytes(uint64_t n_phys) {
-  const uint64_t t = std::max<uint64_t>(probe_tiles(n_phys), compact_tiles(n_phys));
-  return static_cast<size_t>(((t * 8 + 255) / 256) * 256);
+  // as probe_tiles: a bound that never falls as n_phys grows
+  const uint64_t words = bits_words(n_phys);
+  const uint64_t c = std::max<uint64_t>((words + kCompactThreads * 8 - 1) / (kCompactThreads * 8),
+                                        std::min<uint64_t>((words + kCompactThreads - 1) / kCompactThreads, kCompactSumTiles));
+  return static_cast<size_t>(((std::max(probe_tiles(n_phys), c) * 8 + 255) / 256) * 256);
 }
 size_t round256(uint64_t b) { return static_cast<size_t>(((b + 255) / 256) * 256); }
 uint32_t part_tiles(uint64_t n_phys) { return static_cast<uint32_t>((n_phys + kPartTile - 1) / kPartTile); }
@@ -158,7 +162,7 @@ size_t workspace_bytes(uint64_t n_phys) { return ws_layout(n_phys).total; }
 int compact_occupancy() {
   static int occ = [] {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, compact_kernel, kCompactThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, compact_kernel<8>, kCompactThreads, 0);
     return std::max(1, n);
   }();
   return occ;
@@ -465,7 +469,12 @@ dtlg_status launch_probe(const dtlg_filter* f, const uint64_t* words, const uint
     }
   }
   const int cgrid = static_cast<int>(std::min<uint64_t>(tiles, static_cast<uint64_t>(ds->sms) * compact_occupancy()));
-  compact_kernel<<<cgrid, kCompactThreads, 0, stream>>>(c);
+  switch (compact_rows(c.n_words)) {
+    case 1: compact_kernel<1><<<cgrid, kCompactThreads, 0, stream>>>(c); break;
+    case 2: compact_kernel<2><<<cgrid, kCompactThreads, 0, stream>>>(c); break;
+    case 4: compact_kernel<4><<<cgrid, kCompactThreads, 0, stream>>>(c); break;
+    default: compact_kernel<8><<<cgrid, kCompactThreads, 0, stream>>>(c);
+  }
   DTLG_CUDA(cudaGetLastError());
   return DTLG_OK;
 }

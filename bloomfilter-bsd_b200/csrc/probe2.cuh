@@ -6,9 +6,9 @@
 //    thing a warp ever waits for is its own filter loads.  probe_smem_kernel
 //    does the same against a copy of a small filter in shared memory.
 // 2. compact_kernel: turns the bitmask into the ascending position list.  A
-//    tile is 65536 keys (2048 mask words); the tile offset comes from a
-//    decoupled look-back (bounded waits, as in probe.cuh) over a few thousand
-//    status words.  It moves 1/8 byte per key in and 4 bytes per match out,
+//    tile is 8192 to 65536 keys (256 to 2048 mask words, by the batch's size);
+//    the tile offset comes from the tiles' status words, summed at once or by
+//    a decoupled look-back (bounded waits, as in probe.cuh).  It moves 1/8 byte per key in and 4 bytes per match out,
 //    staged per warp in shared memory so the stores are coalesced.
 // The extra traffic against the fused kernel is the bitmask, 2/8 byte per key.
 #pragma once
@@ -21,8 +21,14 @@
 namespace dtlg {
 
 constexpr int kCompactThreads = 256;
-constexpr int kCompactWordsPerThread = 8;
-constexpr uint32_t kCompactTileWords = kCompactThreads * kCompactWordsPerThread;
+// Tiles of 256 mask words (8192 keys) times `rows`: as few rows as give no more
+// than kCompactSumTiles tiles, so that batches of some million keys reach
+// every SM (5 M keys are 77 tiles of 65536) and the offsets are sums; then 8.
+constexpr uint32_t kCompactSumTiles = 1024;
+__host__ __device__ constexpr uint32_t compact_rows(uint64_t n_words) {
+  return n_words <= 256ull * kCompactSumTiles ? 1 : n_words <= 512ull * kCompactSumTiles ? 2
+         : n_words <= 1024ull * kCompactSumTiles ? 4 : 8;
+}
 constexpr uint32_t kMaxGatherCols = 4;
 
 struct CompactArgs {
@@ -117,20 +123,22 @@ probe_smem_kernel(const __grid_constant__ ProbeArgs a, uint32_t* __restrict__ bi
   bits_loop(a, bits, 0, [&](uint32_t key) { return Ops::contains_shared(s_filter, a, key); });
 }
 
-// Ordered compaction.  A tile is kCompactTileWords mask words; warp w of the
-// CTA owns the 256 words w*256 .. w*256+255 of the tile as 8 rows of 32 words
-// (lane l holds word i*32 + l of row i, so every row is one coalesced 128-byte
-// load).  The tile's offset comes from the look-back; the warp's from a CTA
-// scan; each row's from a warp scan.  A row's matches (at most 1024) are
-// first written to a per-warp staging area in shared memory in key order and
-// then stored by the whole warp to consecutive output slots, so the output
-// (and the payload gathers) are coalesced however dense the matches are.
+// Ordered compaction.  A tile is kWarps * ROWS * 32 mask words; warp w of the
+// CTA owns ROWS rows of 32 words (lane l holds word i*32 + l of row i, so every
+// row is one coalesced 128-byte load).  The tile's offset comes from the
+// status words; the warp's from a CTA scan; each row's from a warp scan.  A
+// row's matches (at most 1024) are first written to a per-warp staging area in
+// shared memory in key order and then stored by the whole warp to consecutive
+// output slots, so the output (and the payload gathers) are coalesced however
+// dense the matches are.
+template <int ROWS>
 static __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const __grid_constant__ CompactArgs a) {
   constexpr int kWarps = kCompactThreads / 32;
-  constexpr int kRows = kCompactWordsPerThread;  // rows of 32 words per warp
-  static_assert(kCompactTileWords == kWarps * kRows * 32, "tile = warps x rows x 32 words");
+  constexpr int kRows = ROWS;
+  constexpr uint32_t kTileWords = kCompactThreads * ROWS;
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_warp[kWarps];
+  __shared__ uint32_t s_sum[kWarps];
   __shared__ uint32_t s_excl;
   __shared__ uint32_t s_stage[kWarps][1024];
   const uint32_t lane = threadIdx.x & 31u;
@@ -139,12 +147,13 @@ static __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const _
   ProbeArgs lb{};
   lb.status = a.status;
   lb.err = a.err;
+  const bool by_sum = a.n_tiles <= kCompactSumTiles;
   for (;;) {
     if (threadIdx.x == 0) s_tile = atomicAdd(a.tile_ctr, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= a.n_tiles) break;
-    const uint64_t wbase = static_cast<uint64_t>(tile) * kCompactTileWords + static_cast<uint64_t>(warp) * (kRows * 32);
+    const uint64_t wbase = static_cast<uint64_t>(tile) * kTileWords + static_cast<uint64_t>(warp) * (kRows * 32);
     uint32_t wv[kRows];
     uint32_t c = 0;
 #pragma unroll
@@ -157,6 +166,7 @@ static __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const _
     for (int d = 16; d > 0; d >>= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
     if (lane == 0) s_warp[warp] = c;  // the warp's match count
     __syncthreads();
+    uint32_t agg = 0;
     if (warp == 0) {
       const uint32_t v = lane < kWarps ? s_warp[lane] : 0u;
       uint32_t wi = v;
@@ -165,26 +175,30 @@ static __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const _
         const uint32_t t = __shfl_up_sync(0xffffffffu, wi, d);
         if (lane >= static_cast<uint32_t>(d)) wi += t;
       }
-      const uint32_t agg = __shfl_sync(0xffffffffu, wi, kWarps - 1);
+      agg = __shfl_sync(0xffffffffu, wi, kWarps - 1);
+      if (lane == 0) st_volatile(a.status + tile, ((tile == 0 || by_sum) ? kFlagPrefix : kFlagAgg) | agg);
       if (lane < kWarps) s_warp[lane] = wi - v;
-      uint32_t excl = 0;
-      if (tile == 0) {
-        if (lane == 0) st_volatile(a.status, kFlagPrefix | agg);
-      } else {
-        if (lane == 0) st_volatile(a.status + tile, kFlagAgg | agg);
-        excl = look_back(lb, tile, lane);
-        if (lane == 0) st_volatile(a.status + tile, kFlagPrefix | static_cast<uint32_t>(excl + agg));
-      }
-      if (lane == 0) {
-        s_excl = excl;
-        if (tile == a.n_tiles - 1) {
-          const bool failed = *reinterpret_cast<volatile unsigned int*>(a.err) != 0u;
-          *a.count_out = failed ? ~0ull : static_cast<unsigned long long>(excl) + agg;
+      if (!by_sum) {
+        uint32_t excl = 0;
+        if (tile > 0) {
+          excl = look_back(lb, tile, lane);
+          if (lane == 0) st_volatile(a.status + tile, kFlagPrefix | static_cast<uint32_t>(excl + agg));
         }
+        if (lane == 0) s_excl = excl;
       }
     }
-    __syncthreads();
-    uint32_t pos = s_excl + s_warp[warp];
+    uint32_t excl;
+    if (by_sum) {
+      excl = sum_predecessors(lb, tile, s_sum);  // its barrier also publishes s_warp
+    } else {
+      __syncthreads();
+      excl = s_excl;
+    }
+    if (threadIdx.x == 0 && tile == a.n_tiles - 1) {
+      const bool failed = *reinterpret_cast<volatile unsigned int*>(a.err) != 0u;
+      *a.count_out = failed ? ~0ull : static_cast<unsigned long long>(excl) + agg;
+    }
+    uint32_t pos = excl + s_warp[warp];
     uint32_t* stage = s_stage[warp];
 #pragma unroll
     for (int i = 0; i < kRows; i++) {

@@ -40,3 +40,26 @@ def test_fused_probe_at_shape_edges(case, edge):
             assert got == len(want), (n, pad)
             assert np.array_equal(out[:got].cpu().numpy().view(np.uint32), want), (n, pad)
             assert bool((out[got:] == -1).all()), (n, pad)
+
+
+def test_compaction_at_shape_edges():
+    """The bitmask plan where the compaction's tiles grow from one row of mask
+    words to two, four and eight."""
+    edges = [1 << 23, 1 << 24, 1 << 25]
+    m = N_BUILD * 12
+    ob, f = O.Bloom(4, 1, 1, 1, 4, m), F.bbf_32(m, 4, 1, 1)
+    ref = ob.alloc()
+    ob.insert(ref, keygen.build_keys(N_BUILD, 9))
+    words = torch.zeros(f.alloc_words(), dtype=torch.int64)
+    words[:len(ref)] = torch.from_numpy(ref.view(np.int64))
+    words = words.cuda()
+    pk, _ = keygen.probe_keys(N_BUILD, max(edges) + 32, 0.2, 9)
+    keys, exp = torch.from_numpy(pk.view(np.int32)).cuda(), ob.batch_contains(ref, pk, 0)
+    f.set_probe_options(2, -1)
+    for edge in edges:
+        for n in (edge - 31, edge, edge + 1):
+            want = torch.from_numpy(exp[:np.searchsorted(exp, n)].view(np.int32)).cuda()
+            out = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+            got = f.batch_contains(words, keys, n, out, 0)
+            assert got == len(want) and torch.equal(out[:got], want), n
+            assert bool((out[got:] == -1).all()), n
