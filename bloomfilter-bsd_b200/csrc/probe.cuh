@@ -33,6 +33,12 @@ struct ProbeArgs {
   unsigned int* tile_ctr;       // tile queue head (zeroed)
   unsigned int* err;            // error word (zeroed); bit 0 = wait timed out
   uint32_t n_tiles;
+  // Fused plan, blocking calls (result != null): the CTA that finishes last
+  // clears the words above for the slot's next call and writes the outcome to
+  // host memory (see result_word).
+  unsigned int* done;           // CTAs finished (zeroed)
+  unsigned long long* result;
+  uint32_t ticket;
   Addr addr;
   uint64_t victim_word;         // cuckoo: 32-bit word index of the victim record
   // Block-range pass (two-pass probe only; all zero = off): a key whose block
@@ -50,6 +56,14 @@ struct ProbeArgs {
   // classic Bloom filter: bits per key, and the bit index (h >> shift) & mask
   uint32_t cbf_k, cbf_bit_shift, cbf_bit_mask;
 };
+
+// The outcome of a blocking fused probe in one 64-bit word, so that the host
+// sees all of it or nothing: ticket of the call | error bit | match count
+// (below 2^31 for every batch of the one-round shapes).
+constexpr uint32_t kResultErr = 1u << 31;
+__host__ __device__ constexpr unsigned long long result_word(uint32_t ticket, bool err, uint32_t count) {
+  return static_cast<unsigned long long>(ticket) << 32 | (err ? kResultErr : 0u) | count;
+}
 
 constexpr int kProbeThreads = 256;
 constexpr unsigned long long kFlagAgg = 1ull << 62;
@@ -269,6 +283,30 @@ probe_kernel(const __grid_constant__ ProbeArgs a) {
     __syncthreads();
   }
 }
+  if constexpr (ROUNDS == 1) {
+    if (a.result == nullptr) return;
+    __shared__ bool s_last;
+    __syncthreads();  // the CTA's positions are written
+    if (threadIdx.x == 0) {
+      __threadfence();
+      s_last = a.n_tiles == 1 || atomicAdd(a.done, 1u) == a.n_tiles - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    // every other CTA has finished with the status words
+    if (a.n_tiles > 1)
+      for (uint32_t i = threadIdx.x; i < a.n_tiles; i += blockDim.x) a.status[i] = 0ull;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const bool failed = *reinterpret_cast<volatile unsigned int*>(a.err) != 0u;
+      const unsigned long long n = ld_volatile(a.count_out);
+      *a.tile_ctr = 0u;
+      *a.done = 0u;
+      *a.err = 0u;
+      __threadfence_system();
+      st_volatile(a.result, result_word(a.ticket, failed, static_cast<uint32_t>(n) & ~kResultErr));
+    }
+  }
 
 #endif  // __CUDACC__
 

@@ -92,6 +92,14 @@ int registered_bloom_count();
 constexpr uint32_t kProbeTile = kProbeThreads * 4 * kMaxRounds;
 
 #ifdef __CUDACC__
+// CTAs of `threads` per SM, at least 1 (a query of a few us: its callers keep
+// the answer, which is the same on every call).
+template <class K>
+int occupancy_of(K kernel, int threads) {
+  int n = 0;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0) == cudaSuccess ? std::max(1, n) : 1;
+}
+
 template <class Ops, int MINB>
 struct BitsLaunch {
   static cudaError_t run(const ProbeArgs& a, uint32_t* bits, int or_into, int grid, cudaStream_t s) {
@@ -99,8 +107,7 @@ struct BitsLaunch {
     return cudaGetLastError();
   }
   static int occupancy() {
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, probe_bits_kernel<Ops, MINB>, 256, 0);
+    static const int n = occupancy_of(probe_bits_kernel<Ops, MINB>, 256);
     return n;
   }
   static int local_bytes() {
@@ -126,8 +133,7 @@ struct PairsLaunch {
     return cudaGetLastError();
   }
   static int occupancy() {
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, probe_pairs_kernel<Ops, MINB>, 256, 0);
+    static const int n = occupancy_of(probe_pairs_kernel<Ops, MINB>, 256);
     return n;
   }
   static int local_bytes() {

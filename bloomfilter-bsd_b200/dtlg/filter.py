@@ -43,23 +43,36 @@ class cuckoofilter_config:  # noqa: N801 (reference name)
     addr_mode: int = POWER_OF_TWO
 
 
+_torch_module = None
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
 def _stream():
     torch = _torch()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is not None:  # 0.5 us; a Stream object takes 3.5
+        return C.c_void_p(raw(torch.cuda.current_device()))
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def _dev_ptr(t, name):
-    torch = _torch()
-    if not isinstance(t, torch.Tensor) or not t.is_cuda:
+def _addr(t, name):
+    """The device address of a contiguous CUDA tensor."""
+    if not isinstance(t, _torch().Tensor) or not t.is_cuda:
         raise TypeError(f"{name} must be a CUDA tensor")
     if not t.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
+
+
+def _dev_ptr(t, name):
+    return C.c_void_p(_addr(t, name))
 
 
 def as_device_keys(keys, device=None):
@@ -181,10 +194,11 @@ class filter_base:  # noqa: N801 (reference name)
         """Writes the ascending positions i + match_offset of matching keys to
         match_positions (capacity >= key_cnt); returns the match count."""
         cnt = C.c_uint64(0)
-        check(lib().dtlg_batch_contains(self._h, _dev_ptr(filter_data, "filter_data"), _dev_ptr(keys, "keys"),
-                                        int(key_cnt), _dev_ptr(match_positions, "match_positions"),
-                                        int(match_offset) & 0xFFFFFFFF, C.byref(cnt), _stream()),
-              "batch_contains")
+        st = lib().dtlg_batch_contains(self._h, _addr(filter_data, "filter_data"), _addr(keys, "keys"), int(key_cnt),
+                                       _addr(match_positions, "match_positions"), int(match_offset) & 0xFFFFFFFF,
+                                       C.byref(cnt), _stream())
+        if st:
+            check(st, "batch_contains")
         return cnt.value
 
     def batch_contains_async(self, filter_data, keys, key_cnt, match_positions, match_offset, match_cnt_dev):

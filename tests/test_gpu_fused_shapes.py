@@ -11,7 +11,7 @@ from dtlg import keygen
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
-EDGES = [1024, 256 * 5, 300 << 10, 2 << 20]
+EDGES = [1024, 256 * 5, 148 << 10, 2 << 20]  # one tile, ragged, four keys per thread, four rounds
 N_BUILD = 40000
 
 
@@ -27,6 +27,32 @@ def case(request):
     pk, _ = keygen.probe_keys(N_BUILD, max(EDGES) + 4, 0.3, 8)
     f.set_probe_options(1, -1)
     return f, words.cuda(), torch.from_numpy(pk.view(np.int32)).cuda(), ob.batch_contains(ref, pk, 0)
+
+
+def test_slots_are_clean_between_calls_streams_and_threads(case):
+    """Blocking calls share a bounded set of scratch slots: calls of different
+    sizes, from more threads than slots, each on a stream of its own."""
+    import threading
+    f, words, keys, exp = case
+    bad = []
+
+    def work(t):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(12):
+                n = (1 + 1031 * t + 70001 * i) % (1 << 20) + 1
+                out = torch.empty(n, dtype=torch.int32, device="cuda")
+                want = int(np.searchsorted(exp, n))
+                got = f.batch_contains(words, keys, n, out, 0)
+                if got != want or not np.array_equal(out[:got].cpu().numpy().view(np.uint32), exp[:got]):
+                    bad.append((t, i, n, got, want))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(20)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[:3]
 
 
 @pytest.mark.parametrize("edge", EDGES)
