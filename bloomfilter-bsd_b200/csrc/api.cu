@@ -122,10 +122,9 @@ static_assert(sizeof(WsHeader) == 128, "header is one 128-byte line");
 // n_phys grows, so a workspace sized for more keys always serves fewer).
 uint64_t probe_tiles(uint64_t n_phys) {
   return std::max<uint64_t>((n_phys + kProbeTile - 1) / kProbeTile,
-                            std::min<uint64_t>((n_phys + kProbeThreads - 1) / kProbeThreads, kFusedSumTiles));
+                            std::min<uint64_t>((n_phys + 1023) / 1024, kFusedSumTiles));
 }
-static_assert((kFusedOneKey + kProbeThreads - 1) / kProbeThreads <= kFusedSumTiles &&
-                  (kFusedOneRound + kProbeThreads * 4 - 1) / (kProbeThreads * 4) <= kFusedSumTiles,
+static_assert(kFusedOneKey <= kFusedOneRound && (kFusedOneRound + 1023) / 1024 <= kFusedSumTiles,
               "the status words hold one word per tile of every shape");
 
 // Two-pass layout inside the same workspace: header | status words | bitmask.
@@ -346,6 +345,7 @@ cudaError_t launch_partition(const dtlg_filter* f, const uint32_t* keys_al, uint
   *out = pa;
   return cudaGetLastError();
 }
+
 constexpr size_t kSlotBytes = sizeof(WsHeader) + static_cast<size_t>(kFusedSumTiles) * 8;
 
 // Blocking probes that run on a result slot: the fused plan's one-round shapes.
@@ -377,7 +377,6 @@ cudaError_t wait_for_slot(const ResultSlot& s, cudaStream_t stream, unsigned lon
   *word = *w;
   return cudaSuccess;
 }
-
 
 // Payload columns copied along with the match positions (probe -> gather).
 struct GatherSpec {
@@ -436,12 +435,12 @@ dtlg_status launch_probe(const dtlg_filter* f, const uint64_t* words, const uint
   if (mode == 1) {
     // the fused plan reads Bloom filters that cannot live in L1 without
     // allocating there, as the bitmask plan does (below)
+    a.l1na = (f->bk != nullptr && (f->d.m_actual / 8) > kL1NoAllocBytes) ? 1u : 0u;
     if (slot) {
       a.done = &h->done;
       a.result = slot->host_dev;
       a.ticket = slot->ticket;
     }
-    a.l1na = (f->bk != nullptr && (f->d.m_actual / 8) > kL1NoAllocBytes) ? 1u : 0u;
     DTLG_CUDA(f->pk->probe(a, shape, ds->sms, stream));
     return DTLG_OK;
   }
@@ -1003,6 +1002,7 @@ dtlg_status dtlg_batch_contains(const dtlg_filter* f, const uint64_t* words, con
   if (!f || !match_cnt || (n && (!keys || !out))) return DTLG_ERR_NULL;
   if (dtlg_status st = check_filter_ptr(words)) return st;
   DeviceState* ds = nullptr;
+  if (dtlg_status st = device_state(&ds)) return st;
   cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
   DTLG_CUDA(cudaStreamIsCapturing(stream, &capturing));
   ResultSlot* slot = capturing == cudaStreamCaptureStatusNone ? ds->slots.acquire(kSlotBytes) : nullptr;
@@ -1028,7 +1028,6 @@ dtlg_status dtlg_batch_contains(const dtlg_filter* f, const uint64_t* words, con
   }
   // the other plans: a workspace of their own; its header (error word, count)
   // is copied to the slot's pinned words
-  if (dtlg_status st = device_state(&ds)) return st;
   const size_t ws_bytes = dtlg_probe_workspace_size(n);
   void* ws = nullptr;
   cudaError_t e = cudaMallocFromPoolAsync(&ws, ws_bytes, ds->pool, stream);

@@ -4,8 +4,8 @@
 // write i + match_offset (32-bit wrap) for every matching key index i, in
 // ascending order, and return the count.
 //
-// Shape: CTAs of 256 threads pull tiles of 256 to 4096 keys (fused_shape) from
-// a device counter (so a tile is only ever taken after all earlier tiles were
+// Shape: CTAs of 256 or 1024 threads pull tiles of 1024 or 4096 keys
+// (fused_shape) from a device counter (so a tile is only ever taken after all earlier tiles were
 // taken by running CTAs: the waits below cannot deadlock).  Inside a tile,
 // thread t owns 1 or 4 consecutive keys of each round (4: loaded as one
 // 16-byte vector); matches are ranked with warp ballots and a CTA scan, and
@@ -142,42 +142,43 @@ __device__ __forceinline__ uint32_t sum_predecessors(const ProbeArgs& a, uint32_
 }
 
 // Shape of the fused probe for a batch of n_phys keys: keys per thread and
-// round, rounds per tile, and whether the tile offsets come from
-// sum_predecessors (few tiles) or from look_back.
+// round, rounds per tile, threads per CTA.
 struct FusedShape {
-  uint32_t kpt, rounds, tile, n_tiles;
+  uint32_t kpt, rounds, threads, n_tiles;
 };
 
-// Up to 1024 keys one tile of four keys per thread, which needs no status
-// word; up to kFusedOneKey keys a thread tests one key (tiles of 256 keys), so
-// that a batch of some ten thousand keys already reaches every SM and no
-// thread waits for four gathers one after the other; up to kFusedOneRound keys
-// four (tiles of 1024); beyond, tiles of 4096 keys, whose fewer status words
-// and tickets count more.  Kernel times against tiles of 4096 keys throughout:
-// 60001 keys (zoned u32 w=16 z=4, 225 KiB) 12.7 -> 9.9 us, 900001 keys (u64 w=8
-// s=8 k=8, 8 MiB) 22.7 -> 13.3 us, 1024 keys 4.2 + 1.5 (the zeroing) -> 3.4 us.
+// Up to kFusedOneKey keys a thread tests one key, so that no thread waits for
+// four gathers one after the other, in CTAs of 1024 threads, at most one per
+// SM: few tiles to hand out and sum (blocking calls of 60 000 keys: 16.8 us,
+// with 256-thread CTAs 20.5; 300 000 keys 23.4 against 20.8).  Up to
+// kFusedOneRound keys a thread tests four (tiles of 1024); beyond, tiles of
+// 4096 keys, whose fewer status words and tickets count more.  Kernel times
+// against tiles of 4096 keys throughout, offsets by look-back: 60001 keys
+// (zoned u32 w=16 z=4, 225 KiB) 12.7 -> 9 us, 900001 keys (u64 w=8 s=8 k=8, 8
+// MiB) 22.7 -> 13.3 us, 1024 keys 4.2 + 1.5 (the zeroing) -> 3.4 us.
 constexpr uint32_t kMaxRounds = 4;
-constexpr uint64_t kFusedOneKey = 300ull << 10;
+constexpr uint64_t kFusedOneKey = 148ull << 10;
 constexpr uint64_t kFusedOneRound = 2ull << 20;
 constexpr uint32_t kFusedSumTiles = 2048;  // offsets by sum_predecessors up to this many tiles
 
 __host__ __device__ inline FusedShape fused_shape(uint64_t n_phys) {
   FusedShape s{};
-  s.kpt = n_phys > kProbeThreads * 4 && n_phys <= kFusedOneKey ? 1u : 4u;
+  s.kpt = n_phys <= kFusedOneKey ? 1u : 4u;
+  s.threads = s.kpt == 1 ? 1024u : static_cast<uint32_t>(kProbeThreads);
   s.rounds = n_phys <= kFusedOneRound ? 1u : kMaxRounds;
-  s.tile = static_cast<uint32_t>(kProbeThreads) * s.kpt * s.rounds;
-  s.n_tiles = static_cast<uint32_t>((n_phys + s.tile - 1) / s.tile);
+  const uint32_t tile = s.threads * s.kpt * s.rounds;
+  s.n_tiles = static_cast<uint32_t>((n_phys + tile - 1) / tile);
   return s;
 }
 
 // Ops::contains(const ProbeArgs&, uint32_t key) -> bool, safe for any key
 // value (block / bucket indexes are always inside the filter).  KPT keys per
 // thread and round, ROUNDS rounds per tile.
-template <class Ops, int KPT, int ROUNDS>
-__global__ void __launch_bounds__(kProbeThreads)
+template <class Ops, int KPT, int ROUNDS, int THREADS>
+__global__ void __launch_bounds__(THREADS)
 probe_kernel(const __grid_constant__ ProbeArgs a) {
-  constexpr uint32_t kRoundKeys = kProbeThreads * KPT;
-  constexpr uint32_t kWarps = kProbeThreads / 32;
+  constexpr uint32_t kRoundKeys = THREADS * KPT;
+  constexpr uint32_t kWarps = THREADS / 32;
   static_assert(ROUNDS * kWarps <= 32, "one warp scans the warp totals");
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_wtot[ROUNDS * kWarps];
@@ -282,7 +283,6 @@ probe_kernel(const __grid_constant__ ProbeArgs a) {
     if (a.n_tiles <= gridDim.x) break;  // one tile per CTA
     __syncthreads();
   }
-}
   if constexpr (ROUNDS == 1) {
     if (a.result == nullptr) return;
     __shared__ bool s_last;
@@ -307,6 +307,7 @@ probe_kernel(const __grid_constant__ ProbeArgs a) {
       st_volatile(a.result, result_word(a.ticket, failed, static_cast<uint32_t>(n) & ~kResultErr));
     }
   }
+}
 
 #endif  // __CUDACC__
 

@@ -148,15 +148,13 @@ struct FusedLaunch {
   // tile waits only for tiles taken before it), the resident CTAs beyond.
   static cudaError_t run(const ProbeArgs& a, const FusedShape& shape, int sms, cudaStream_t s) {
     if (shape.kpt == 1) {
-      probe_kernel<Ops, 1, 1><<<a.n_tiles, kProbeThreads, 0, s>>>(a);
+      probe_kernel<Ops, 1, 1, 1024><<<a.n_tiles, 1024, 0, s>>>(a);
     } else if (shape.rounds == 1) {
-      probe_kernel<Ops, 4, 1><<<a.n_tiles, kProbeThreads, 0, s>>>(a);
+      probe_kernel<Ops, 4, 1, kProbeThreads><<<a.n_tiles, kProbeThreads, 0, s>>>(a);
     } else {
-      constexpr auto kernel = probe_kernel<Ops, 4, kMaxRounds>;
-      int occ = 0;
-      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kProbeThreads, 0);
-      if (e != cudaSuccess) return e;
-      const uint32_t resident = static_cast<uint32_t>(sms) * static_cast<uint32_t>(std::max(1, occ));
+      constexpr auto kernel = probe_kernel<Ops, 4, kMaxRounds, kProbeThreads>;
+      static const int occ = occupancy_of(kernel, kProbeThreads);
+      const uint32_t resident = static_cast<uint32_t>(sms) * static_cast<uint32_t>(occ);
       kernel<<<std::min(a.n_tiles, resident), kProbeThreads, 0, s>>>(a);
     }
     return cudaGetLastError();
