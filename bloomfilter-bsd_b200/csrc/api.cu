@@ -322,6 +322,7 @@ cudaError_t launch_partition(const dtlg_filter* f, const uint32_t* keys_al, uint
   pa.addr = f->d.addr;
   pa.block_mul = mul_const(f->xk ? 1 : 0);
   partition_ranges(f, &pa.range_log2, &pa.n_ranges);
+  pa.range_shift = 32 - clog2(f->d.addr.block_cnt) + pa.range_log2;  // POW2 only
   pa.n_tiles = part_tiles(n_phys);
   part_segments(n_phys - pre, f->d.addr.block_cnt, pa.range_log2, pa.n_ranges, &pa.seg_cap, &pa.last_cap);
   pa.hdr = reinterpret_cast<PartHeader*>(wsb + lay.part_off);

@@ -68,6 +68,7 @@ struct PartArgs {
   uint32_t pre;
   Addr addr;
   uint32_t range_log2;      // a range is 2^range_log2 consecutive blocks
+  uint32_t range_shift;     // POW2: range = block hash >> range_shift (32: one range)
   uint32_t n_ranges;
   uint32_t n_tiles;
   uint32_t block_mul;       // the family constant of the block hash (C[0]; C[1]: blocked cuckoo)
@@ -100,125 +101,148 @@ __device__ __forceinline__ uint32_t key_range(uint32_t key, const PartArgs& a) {
 }
 
 // key_range with the addressing mode fixed at compile time (block_index
-// branches on it at run time).
+// branches on it at run time): under POW2 the top bits of the block hash (the
+// funnel shift gives 0 for the shift of 32 that a single range has).
 template <bool MAGIC>
 __device__ __forceinline__ uint32_t key_range_of(uint32_t key, const PartArgs& a) {
-  return block_index_of<MAGIC>(key * a.block_mul, a.addr) >> a.range_log2;
+  const uint32_t h = key * a.block_mul;
+  if constexpr (MAGIC) return block_index_of<true>(h, a.addr) >> a.range_log2;
+  return __funnelshift_rc(h, 0u, a.range_shift);
 }
 
 // Shared memory of one scatter CTA.
 struct ScatterSmem {
   unsigned long long kv[kPartTile];    // the tile sorted by range: key | tile-local index << 32
-  uint32_t cur[kMaxRanges];            // counts, then the placement cursor
+  uint32_t cnt[kMaxRanges];            // keys per range
+  uint32_t start[kMaxRanges];          // sorted slot of the range's first key
   uint32_t lim[kMaxRanges];            // sorted slots below this go to the segment, the rest overflow
   unsigned long long dst[kMaxRanges];  // pair index of sorted slot 0 for the range's run
   uint32_t valid;
+  uint32_t any_over;                   // some run of the tile does not fit
   unsigned long long over;
 };
 
-// One pass: per tile, count the keys of every range, reserve the tile's run of
-// each range in its segment (one global atomic per tile and range), sort the
-// tile by range in shared memory and write every run with consecutive
-// addresses.  Shared memory holds the sorted keys with their 12-bit tile
-// positions, one 64-bit word each (32 KiB).  The kernel is bound by instruction issue, so the
-// addressing mode is a template parameter (POW2 or MAGIC, chosen by the
-// launch), the tile's index arithmetic is 32-bit, a key's range is computed
-// once for the count and the placement (kept as bytes), and each range's
-// destination base and slot limit are computed once per tile.  512 threads of
-// 8 keys each, four CTAs per SM (2^28 keys over 64 ranges of a 512 MiB POW2
-// filter: 959 us with 256 threads of 16 keys and run-time addressing, 896 us
-// so).
-template <bool MAGIC, int THREADS>
+// One pass: per tile, count the keys of every range (the counting atomic's
+// result is the key's rank in its run), reserve the tile's run of each range
+// in its segment (one global atomic per tile and range), sort the tile by
+// range in shared memory and write every run with consecutive addresses.
+// Shared memory holds the sorted keys with their 12-bit tile positions, one
+// 64-bit word each (32 KiB).  The kernel is bound by instruction issue and
+// shared-memory wavefronts, so the addressing mode is a template parameter
+// (POW2 or MAGIC, chosen by the launch), tiles of valid keys take no test per
+// key (FULL), runs that all fit take none at the write-out, and the ranks are
+// kept, two per register.  512 threads of 8 keys each, four CTAs per SM.  2^28
+// keys over 64 ranges (512 MiB POW2 filter): 899 us with a range by
+// multiplication, a second atomic per key and the tests, 782 us so (LSU data
+// pipe 76 % busy, 36 warp instructions per 32 keys against 77).
+template <bool MAGIC, int THREADS, bool FULL>
 __device__ __forceinline__ void scatter_tile(const PartArgs& a, uint32_t tile, ScatterSmem& S) {
   constexpr int kVecs = static_cast<int>(kPartTile) / THREADS / 4;  // key vectors per thread
   static_assert(kVecs * 4 * THREADS == static_cast<int>(kPartTile), "tile");
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t tile_pos = static_cast<uint64_t>(tile) * kPartTile;  // physical index of the tile's key 0
   // valid keys of this tile: tile-local indexes [lo, hi)
-  const uint32_t lo = tile_pos < a.pre ? static_cast<uint32_t>(a.pre - tile_pos) : 0u;
-  const uint32_t hi = a.n_phys - tile_pos < kPartTile ? static_cast<uint32_t>(a.n_phys - tile_pos) : kPartTile;
-  const uint4* t4 = reinterpret_cast<const uint4*>(a.keys_al) + tile_pos / 4;
+  const uint32_t lo = FULL || tile_pos >= a.pre ? 0u : static_cast<uint32_t>(a.pre - tile_pos);
+  const uint32_t hi =
+      FULL || a.n_phys - tile_pos >= kPartTile ? kPartTile : static_cast<uint32_t>(a.n_phys - tile_pos);
+  const uint4* t4 = reinterpret_cast<const uint4*>(a.keys_al) + tile_pos / 4 + threadIdx.x;
+  auto valid = [&](uint32_t li) { return FULL || (li >= lo && li < hi); };
   // the keys are read twice: for the counts and, from L2, for the placement
-  // (holding them across the scan would not fit 32 registers); their ranges
-  // are kept, four bytes per register
-  uint32_t rr[kVecs];
+  uint32_t rank[kVecs * 2];  // two 16-bit ranks per register
   {
     uint4 kv[kVecs];
 #pragma unroll
     for (int i = 0; i < kVecs; i++) {
       const uint32_t li = (i * THREADS + threadIdx.x) * 4;
-      kv[i] = li < hi ? __ldcg(t4 + li / 4) : make_uint4(0, 0, 0, 0);
+      kv[i] = FULL || li < hi ? __ldcg(t4 + i * THREADS) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int i = 0; i < kVecs; i++) {
       const uint32_t li = (i * THREADS + threadIdx.x) * 4;
       const uint32_t k[4] = {kv[i].x, kv[i].y, kv[i].z, kv[i].w};
-      rr[i] = 0;
+      uint32_t rk[4];
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint32_t r = key_range_of<MAGIC>(k[q], a);
-        rr[i] |= r << (8 * q);
-        if (li + q >= lo && li + q < hi) atomicAdd(&S.cur[r], 1u);
-      }
+      for (int q = 0; q < 4; q++) rk[q] = valid(li + q) ? atomicAdd(&S.cnt[key_range_of<MAGIC>(k[q], a)], 1u) : 0u;
+      rank[2 * i] = rk[0] | rk[1] << 16;
+      rank[2 * i + 1] = rk[2] | rk[3] << 16;
     }
   }
   __syncthreads();
+  uint32_t c[2], g[2], lb[2];
   if (threadIdx.x < 32) {
-    // tile-local run starts (exclusive scan, two ranges per lane), the runs'
-    // slots in their segments, and per range the destination of sorted slot
-    // 0 and the first sorted slot that no longer fits the segment
-    const uint32_t r0 = lane * 2, r1 = lane * 2 + 1;
-    const uint32_t c0 = S.cur[r0], c1 = S.cur[r1];
-    const uint32_t pair = c0 + c1;
+    // tile-local run starts (exclusive scan, two ranges per lane) and the
+    // runs' slots in their segments (used after the placement)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      c[h] = S.cnt[lane * 2 + h];
+      g[h] = c[h] ? atomicAdd(&a.hdr->fill[lane * 2 + h], c[h]) : 0u;
+    }
+    const uint32_t pair = c[0] + c[1];
     uint32_t incl = pair;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const uint32_t x = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= static_cast<uint32_t>(d)) incl += x;
     }
-    const uint32_t b0 = incl - pair;
+    lb[0] = incl - pair;
+    lb[1] = lb[0] + c[0];
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const uint32_t r = h ? r1 : r0, c = h ? c1 : c0, lb = h ? b0 + c0 : b0;
-      const uint32_t g = c ? atomicAdd(&a.hdr->fill[r], c) : 0u;
-      const uint64_t cap = r + 1 < a.n_ranges ? a.seg_cap : a.last_cap;
-      const uint64_t room = g < cap ? cap - g : 0;
-      S.cur[r] = lb;
-      S.lim[r] = lb + static_cast<uint32_t>(room < c ? room : c);
-      S.dst[r] = static_cast<uint64_t>(r) * a.seg_cap + g - lb;
-    }
+    for (int h = 0; h < 2; h++) S.start[lane * 2 + h] = lb[h];
     if (lane == 31) S.valid = incl;
   }
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < kVecs; i++) {
     const uint32_t li = (i * THREADS + threadIdx.x) * 4;
-    const uint4 x = li < hi ? __ldcs(t4 + li / 4) : make_uint4(0, 0, 0, 0);
+    const uint4 x = FULL || li < hi ? __ldcs(t4 + i * THREADS) : make_uint4(0, 0, 0, 0);
     const uint32_t k[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      if (li + q >= lo && li + q < hi) {
-        const uint32_t slot = atomicAdd(&S.cur[(rr[i] >> (8 * q)) & 0xffu], 1u);
-        S.kv[slot] = static_cast<unsigned long long>(li + q) << 32 | k[q];
-      }
+      const uint32_t rk = q & 1 ? rank[2 * i + q / 2] >> 16 : rank[2 * i + q / 2] & 0xffffu;
+      if (valid(li + q))
+        S.kv[S.start[key_range_of<MAGIC>(k[q], a)] + rk] = static_cast<unsigned long long>(li + q) << 32 | k[q];
     }
   }
+  if (threadIdx.x < 32) {
+    // per range the destination of sorted slot 0 and the first sorted slot
+    // that no longer fits the segment; the counts start anew
+    bool over = false;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint32_t r = lane * 2 + h;
+      const uint64_t cap = r + 1 < a.n_ranges ? a.seg_cap : a.last_cap;
+      const uint64_t room = g[h] < cap ? cap - g[h] : 0;
+      S.lim[r] = lb[h] + static_cast<uint32_t>(room < c[h] ? room : c[h]);
+      S.dst[r] = static_cast<uint64_t>(r) * a.seg_cap + g[h] - lb[h];
+      S.cnt[r] = 0;
+      over |= room < c[h];
+    }
+    over = __any_sync(0xffffffffu, over);
+    if (lane == 0) S.any_over = over;
+  }
   __syncthreads();
-  // the placement cursors are not read below: clear them for the next tile
-  // (the barrier after the write-out orders this before its counts)
-  if (threadIdx.x < kMaxRanges) S.cur[threadIdx.x] = 0;
-  const uint32_t nv = S.valid;
   const uint32_t pos0 = static_cast<uint32_t>(tile_pos - a.pre);  // logical position of tile index 0 (mod 2^32)
-  for (uint32_t sl = threadIdx.x; sl < nv; sl += THREADS) {
-    const unsigned long long kv = S.kv[sl];
-    const uint32_t key = static_cast<uint32_t>(kv);
-    const uint32_t r = key_range_of<MAGIC>(key, a);
-    const uint2 pr = make_uint2(key, pos0 + static_cast<uint32_t>(kv >> 32));
-    if (sl < S.lim[r]) {
-      __stcs(a.pairs + (S.dst[r] + sl), pr);
-    } else {
-      atomicOr(&S.over, 1ull << r);
-      if (a.spill) a.spill[atomicAdd(&a.hdr->spill_cnt, 1u)] = pr;
+  if (FULL && S.any_over == 0) {
+#pragma unroll 4
+    for (uint32_t j = 0; j < kPartTile / THREADS; j++) {
+      const uint32_t sl = j * THREADS + threadIdx.x;
+      const unsigned long long kv = S.kv[sl];
+      const uint32_t key = static_cast<uint32_t>(kv);
+      __stcs(a.pairs + (S.dst[key_range_of<MAGIC>(key, a)] + sl), make_uint2(key, pos0 + static_cast<uint32_t>(kv >> 32)));
+    }
+  } else {
+    const uint32_t nv = S.valid;
+    for (uint32_t sl = threadIdx.x; sl < nv; sl += THREADS) {
+      const unsigned long long kv = S.kv[sl];
+      const uint32_t key = static_cast<uint32_t>(kv);
+      const uint32_t r = key_range_of<MAGIC>(key, a);
+      const uint2 pr = make_uint2(key, pos0 + static_cast<uint32_t>(kv >> 32));
+      if (sl < S.lim[r]) {
+        __stcs(a.pairs + (S.dst[r] + sl), pr);
+      } else {
+        atomicOr(&S.over, 1ull << r);
+        if (a.spill) a.spill[atomicAdd(&a.hdr->spill_cnt, 1u)] = pr;
+      }
     }
   }
   __syncthreads();
@@ -227,13 +251,17 @@ __device__ __forceinline__ void scatter_tile(const PartArgs& a, uint32_t tile, S
 template <bool MAGIC, int THREADS = kPartThreads>
 static __global__ void __launch_bounds__(THREADS, 2048 / THREADS) part_scatter_kernel(const __grid_constant__ PartArgs a) {
   __shared__ ScatterSmem S;
-  // The counters start at zero; each tile clears them again for the next one
-  // while it writes its runs out, so a tile needs no barrier of its own for it.
-  if (threadIdx.x < kMaxRanges) S.cur[threadIdx.x] = 0;
+  // The counters start at zero; each tile clears them again for the next one.
+  if (threadIdx.x < kMaxRanges) S.cnt[threadIdx.x] = 0;
   if (threadIdx.x == 0) S.over = 0;
   __syncthreads();
   for (uint32_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
-    scatter_tile<MAGIC, THREADS>(a, tile, S);
+    const uint64_t pos = static_cast<uint64_t>(tile) * kPartTile;
+    if (pos >= a.pre && a.n_phys - pos >= kPartTile) {
+      scatter_tile<MAGIC, THREADS, true>(a, tile, S);
+    } else {
+      scatter_tile<MAGIC, THREADS, false>(a, tile, S);
+    }
     if (threadIdx.x == 0) {
       // S.over is next written in the next tile's write-out, three barriers on
       a.tile_overflow[tile] = S.over;
