@@ -222,29 +222,24 @@ constexpr uint64_t kSmemMaxBytes = 192ull << 10;
 // 112 Gkeys/s; not allocating, 1-8 MiB: 128.7).
 constexpr uint64_t kL1NoAllocBytes = 256ull << 10;
 
-// Blocked Bloom filters just beyond the single-pass limit whose words the
-// hash picks one by one (s < w), or of one word per block, and zoned u32
-// filters of 192 MiB: the bitmask plan in its block-range passes with the
-// 32-register variant beats the partitioned plan.  B200, 2^27 probes, Gkeys/s,
-// bitmask vs partition:
-//   u32 w=16 s=1 k=4    192 / 224 / 256 MiB: 106.1 / 98.1 / 90.4 vs 81.9 / 82.9 / 83.3
-//   u64 w=8 s=2 k=8     192 MiB: 75.9 vs 64.0
-//   u32 w=1 k=4         168 / 192 MiB: 136.2 / 119.5 vs 102.7 / 104.1 (256: 93.6 vs 105.9)
-//   zoned u32 w=16 z=2  192 / 256 MiB: 105.0 / 89.6 vs 97.9 / 100.6
-// Layouts that test half a block before loading the rest (s >= w with blocks
-// of >= 64 bytes) and zoned u64 ones probe faster partitioned from 160 MiB on
-// (u64 w=8 s=8 k=8 168 / 192 MiB: 89.8 / 85.5 vs 91.2 / 88.9; zoned u64 w=8
-// z=4 192 MiB: 74.6 vs 83.9; z=2 256 MiB: 87.8 vs 94.4), as do 32-byte blocks
-// (u64 w=4 s=4 k=8, 168 MiB: 83.9 vs 89.7).
+// Filters just beyond the single-pass limit that the bitmask plan still probes
+// faster, in its block-range passes, than the partitioned plan: layouts that
+// pick their words from the whole block (s = 1, and s = 2 of 16 u32 words), and
+// u32 of one word per block.  us for 2^27 probes, bitmask / partitioned, at
+// 168, 192 and 224 MiB: u32 w=16 s=1 k=4 1115/1282, 1222/1307, 1324/1286; s=2
+// 1115/1180, 1246/1266, 1338/1188; u32 w=1 k=4 940/1026, 1093/1039; at 168 MiB
+// s=1 of u32 w=2 to 8 and u64 w=4, 8 the bitmask plan is 5 to 10 % faster, at
+// 200 MiB 2 % slower.  The others are partitioned from 160 MiB on (at 168 MiB
+// u64 w=8 s=4 1878/1230, u32 w=16 s=8 1497/1178, u64 w=8 s=2 1645/1620, u64 w=1
+// 1229/1020, u32 w=4 1061/1033, zoned u32 w=16 z=2 1144/1093, z=4 1241/1174).
 bool bitmask_band(const dtlg_filter* f) {
-  if (f->d.kind != Kind::kBloom && f->d.kind != Kind::kZoned) return false;
+  if (f->d.kind != Kind::kBloom) return false;
   const uint64_t fbytes = (f->d.m_actual + 7) / 8;
-  const uint64_t block_bytes = static_cast<uint64_t>(f->d.w) * f->d.word_bytes;
   if (fbytes <= (160ull << 20)) return false;
   // the limits leave room for MAGIC sizes, which round a request up
-  if (f->d.kind == Kind::kZoned) return f->d.word_bytes == 4 && fbytes <= (224ull << 20);
-  if (f->d.s < f->d.w) return fbytes <= (264ull << 20);
-  return block_bytes < 32 && fbytes <= (240ull << 20);
+  const bool u32 = f->d.word_bytes == 4;
+  if (u32 && f->d.w == 16 && f->d.s <= 2) return fbytes <= (200ull << 20);
+  return f->d.s == 1 && (u32 || f->d.w > 1) && fbytes <= (180ull << 20);
 }
 
 int probe_plan(const dtlg_filter* f, uint64_t n) {
@@ -266,24 +261,62 @@ int probe_plan(const dtlg_filter* f, uint64_t n) {
   return mode;
 }
 
+// Cuckoo tables that hit L1 on part of the loads only are probed key by key:
+// with more loads in flight the lines are gone before they are used again.  us
+// for 2^26 probes, key by key / together, at 64, 256, 320, 512 and 1024 KiB:
+// t=8 280/274 315/336 381/421 458/466 510/473, t=32 245/268 353/361 398/415
+// 458/463 508/510, t=16 303/258 331/316 369/383 461/458 509/485; 12-bit tags
+// gain throughout (390/390 441/436 499/489 582/571 634/608).
+bool cuckoo_keys_together(const dtlg_filter* f) {
+  const uint64_t kib = f->d.m_actual >> 13;
+  return f->d.t == 12 || kib > 512 || (kib <= 224 && f->d.t != 32);
+}
+
+// Variant of the bitmask kernel, 0 = 6 CTAs per SM (40 registers) or 1 = 4 (64
+// registers), for a filter read in one pass.  us for 2^26 probes, 0 / 1, in L2
+// (8 MiB), at 64 and at 96 MiB, where more of the loads come from the far half
+// of the L2 or from DRAM and more warps in flight hide them:
+//   u64 w=8 s=8 k=8      342/382 383/454 506/595     u32 w=16 z=2   315/320 336/360 492/513
+//   u32 w=16 s=8         336/344 372/395 500/527     u64 w=8 s=2    599/672 638/690 793/797
+//   u64 w=8 z=2          338/333 366/379 495/514     u64 w=8 z=4    434/410 441/464 522/603
+//   u64 w=8 s=4          469/459 480/503 539/625     u32 w=16 z=4   375/374 378/394 502/521
+//   u32 w=16 s=1 k=4     444/442 450/432 489/498     u64 w=4 s=4    364/357 385/379 480/520
+//   u32 w=1 k=4          289/293 299/291 503/492     u64 w=16 k=16  717/611 723/659 784/761
+// (an 8-CTA, 32-register form was slower than 0 everywhere but for u64 w=8 s=2
+// beyond 64 MiB, 723 at 96, and z=4 and s=4 at 80 to 96).  Bloom layouts whose
+// kernel 0 spills take kernel 1.
+int bits_variant_for(const dtlg_filter* f) {
+  if (f->ck) {
+    // two-pass tables miss L2 more (t=16 b=4, 142 MiB: 660 / 722; t=12 b=4, 106
+    // MiB 754 / 802); in one pass only 16-bit tags gain (510 / 532, 12-bit 640
+    // / 627, 8-bit 481 / 479, 32-bit 575 / 544), 12-bit ones up to 512 KiB (364
+    // / 384 at 16 KiB, 436 / 450 at 256)
+    return probe_passes(f) > 1 || f->d.t == 16 || (f->d.t == 12 && f->d.m_actual <= (512ull << 13)) ? 0 : 1;
+  }
+  if (!f->bk || f->d.k > 8) return 1;
+  const uint64_t mib = f->d.m_actual >> 23;
+  const uint32_t block = f->d.w * f->d.word_bytes, s = f->d.s, w = f->d.w;
+  const bool zoned = f->d.kind == Kind::kZoned, u32 = f->d.word_bytes == 4;
+  if (block == 32) return mib >= 68 && mib <= 116 ? 0 : 1;
+  if (block != 64) return 1;
+  if (zoned) return (u32 && f->d.z == 2) || mib >= 60 ? 0 : 1;
+  if (s >= w) return 0;
+  if (u32) return s * 2 == w || (mib >= 88 && mib <= 116) ? 0 : 1;
+  if (s == 1) return mib >= 72 && mib <= 116 ? 0 : 1;
+  return s == 2 ? (mib <= 88 ? 0 : 1) : (mib >= 60 ? 0 : 1);
+}
+
 // Register-budget variant of the bitmask / pair kernels for plan `mode`: the
-// caller's, else 0 for the bitmask plan in the band above and for the pair
-// probe of Bloom filters, else 1.  Pair probe, v0 against v1, Gkeys/s:
-// u64 w=8 s=8 k=8 at 192 / 256 / 512 MiB 88.9 / 91.5 / 84.9 against 84.8 /
-// 85.3 / 80.4 with 32 MiB ranges, 92.2 / 94.3 / 89.0 against 89.7 / 92.1 /
-// 90.5 with 8 MiB ranges; zoned u64 w=8 z=2 at 256 / 384 MiB 94.4 / 91.1
-// against 92.7 / 88.3.
-// A 32-register bitmask kernel that spills (local memory per thread, from
-// cudaFuncGetAttributes; -Xptxas -v: 19 layouts) gives way to the 64-register
-// one: u64 w=1 k=16 at 200 MiB, 2^27 probes, spilling v0 65.1 against v1 69.3
-// Gkeys/s.  The pair probe keeps v0 where it spills (7 layouts, all k >= 12):
-// its spills cost less than the halved occupancy of v1 (u64 w=8 s=8 k=16 at
-// 512 MiB: 83.0 against 79.7; u64 w=4 s=4 k=16 at 192 MiB: 89.7 against 87.5).
+// caller's, else as above for the bitmask plan in one pass, 0 in the band
+// above and for the pair probe of Bloom filters, 1 for that of the others.
+// Pair probe (2^27 probes, 512 MiB, 8 / 6 / 4 CTAs per SM, us): u64 w=8 s=8 k=8
+// 1195 / 1243 / 1294; the form of 8 keeps its lead where it spills (7 layouts,
+// all k >= 12: u64 w=8 s=8 k=16 at 512 MiB 83.0 against 79.7 Gkeys/s).
 int probe_variant(const dtlg_filter* f, int mode) {
   if (f->bits_variant >= 0 && f->bits_variant < kBitsVariants) return f->bits_variant;
   if (mode == 3) return (f->d.kind == Kind::kBloom || f->d.kind == Kind::kZoned) ? 0 : 1;
-  int v = bitmask_band(f) ? 0 : 1;
-  if (v == 0) {
+  int v = bitmask_band(f) ? 0 : bits_variant_for(f);
+  if (v == 0 && f->bk) {
     const occ_fn spill = f->pk->bits_local_bytes[0];
     if (spill && spill() != 0) v = 1;
   }
@@ -460,6 +493,7 @@ dtlg_status launch_probe(const dtlg_filter* f, const uint64_t* words, const uint
     // cuckoo buckets 75.6 -> 47.9, blocked cuckoo (128 MiB) 102.1 -> 98.9,
     // classic Bloom unchanged.
     a.l1na = (f->bk != nullptr && (f->d.m_actual / 8) > kL1NoAllocBytes) ? 1u : 0u;
+    a.together = cuckoo_keys_together(f) ? 1u : 0u;
     // match bitmask, in block-range passes over large filters (each pass
     // probes only the keys whose block lies in its range, so the concurrently
     // touched part of the filter stays within the GPU's address-translation reach)

@@ -77,51 +77,77 @@ struct CuckooOps {
     tag += (tag == 0u);                          // :184
   }
 
-  // Does bucket i hold `tag`?  Reads the bucket's bytes with aligned loads.
-  __device__ __forceinline__ static bool bucket_has(const void* table, uint32_t i, uint32_t tag) {
+  // A bucket's bytes, read with aligned loads: one word, or the two aligned
+  // 32-bit words that hold a bucket of 1, 2, 3 or 6 bytes and the bucket's
+  // first bit in them.
+  struct Bucket {
+    unsigned long long x = 0;
+    unsigned long long y = 0;  // buckets of 16 bytes: the second half
+    uint32_t sh = 0;
+  };
+  __device__ __forceinline__ static Bucket load(const void* table, uint32_t i) {
     const uint64_t o = static_cast<uint64_t>(i) * kBPB;
     const unsigned char* t8 = static_cast<const unsigned char*>(table);
-    bool hit = false;
+    Bucket b;
     if constexpr (kBPB == 16) {
-      const uint4 x = __ldg(reinterpret_cast<const uint4*>(t8 + o));
-      hit = (x.x == tag) | (x.y == tag) | (x.z == tag) | (x.w == tag);
+      const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(t8 + o));
+      b.x = v.x;
+      b.y = v.y;
     } else if constexpr (kBPB == 8) {
-      const unsigned long long x = __ldg(reinterpret_cast<const unsigned long long*>(t8 + o));
-#pragma unroll
-      for (int j = 0; j < kB; j++) hit |= ((x >> (kT * j)) & Cfg::kTagMask) == tag;
+      b.x = __ldg(reinterpret_cast<const unsigned long long*>(t8 + o));
     } else if constexpr (kBPB == 4) {
-      const uint32_t x = __ldg(reinterpret_cast<const unsigned int*>(t8 + o));
-#pragma unroll
-      for (int j = 0; j < kB; j++) hit |= ((x >> (kT * j)) & Cfg::kTagMask) == tag;
+      b.x = __ldg(reinterpret_cast<const unsigned int*>(t8 + o));
     } else {
-      // 1, 2, 3 or 6 bytes: at most two aligned 32-bit words hold the bucket
       const uint64_t a4 = o & ~3ull;
-      const uint32_t sh = static_cast<uint32_t>(o & 3u) * 8u;
+      b.sh = static_cast<uint32_t>(o & 3u) * 8u;
       const unsigned int* w = reinterpret_cast<const unsigned int*>(t8 + a4);
-      unsigned long long x = __ldg(w);
-      if constexpr (kBPB > 2) x |= static_cast<unsigned long long>(__ldg(w + 1)) << 32;
+      b.x = __ldg(w);
+      if constexpr (kBPB > 2) b.x |= static_cast<unsigned long long>(__ldg(w + 1)) << 32;
+    }
+    return b;
+  }
+  // Does the bucket hold `tag`?  A Bucket{} holds none (no tag is 0).
+  __device__ __forceinline__ static bool holds(const Bucket& b, uint32_t tag) {
+    bool hit = false;
 #pragma unroll
-      for (int j = 0; j < kB; j++) hit |= ((x >> (sh + kT * j)) & Cfg::kTagMask) == tag;
+    for (int j = 0; j < kB; j++) {
+      const unsigned long long x = kBPB == 16 && j >= kB / 2 ? b.y : b.x;
+      const int at = kBPB == 16 ? kT * (j % (kB / 2 > 0 ? kB / 2 : 1)) : kT * j;
+      hit |= (static_cast<uint32_t>(x >> (b.sh + at)) & Cfg::kTagMask) == tag;
     }
     return hit;
   }
 
-  // cuckoofilter_logic.hpp:346-362
-  __device__ __forceinline__ static bool contains(const ProbeArgs& a, uint32_t key) {
-    uint32_t i1, tag;
-    index_tag(key, a.addr, i1, tag);
-    const uint32_t i2 = cuckoo_alt(i1, tag, a.addr);
+  // cuckoofilter_logic.hpp:346-362 for N keys at once: the buckets of all of
+  // them are loaded before any is tested.  One key after the other, each
+  // bucket behind a branch of its own, a thread had one load in flight, and
+  // the probe ran at the loads' latency.  Bit q of the result: key q matches.
+  template <int N>
+  __device__ __forceinline__ static uint32_t contains_n(const ProbeArgs& a, const uint32_t (&key)[N]) {
+    uint32_t i1[N], i2[N], tag[N];
+    Bucket b1[N], b2[N];
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+      index_tag(key[q], a.addr, i1[q], tag[q]);
+      i2[q] = cuckoo_alt(i1[q], tag[q], a.addr);
+      // block-range pass: only the buckets this pass owns (the result is the
+      // OR over all passes)
+      if (!a.range_on || (i1[q] >= a.blk_lo && i1[q] < a.blk_hi)) b1[q] = load(a.filter, i1[q]);
+      if (!a.range_on || (i2[q] >= a.blk_lo && i2[q] < a.blk_hi)) b2[q] = load(a.filter, i2[q]);
+    }
     const unsigned int* v = static_cast<const unsigned int*>(a.filter) + a.victim_word;
     const uint32_t vi = __ldg(v), vt = __ldg(v + 1), vu = __ldg(v + 2) & 0xffu;
-    const bool in_victim = vu && tag == vt && (i1 == vi || i2 == vi);
-    if (a.range_on) {
-      // block-range pass: only the buckets this pass owns (the result is the OR
-      // over all passes)
-      const bool r1 = i1 >= a.blk_lo && i1 < a.blk_hi;
-      const bool r2 = i2 >= a.blk_lo && i2 < a.blk_hi;
-      return in_victim | (r1 && bucket_has(a.filter, i1, tag)) | (r2 && bucket_has(a.filter, i2, tag));
+    uint32_t hits = 0;
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+      const bool in_victim = vu && tag[q] == vt && (i1[q] == vi || i2[q] == vi);
+      hits |= (in_victim | holds(b1[q], tag[q]) | holds(b2[q], tag[q]) ? 1u : 0u) << q;
     }
-    return in_victim | bucket_has(a.filter, i1, tag) | bucket_has(a.filter, i2, tag);
+    return hits;
+  }
+  __device__ __forceinline__ static bool contains(const ProbeArgs& a, uint32_t key) {
+    const uint32_t k[1] = {key};
+    return contains_n<1>(a, k) != 0u;
   }
 
   // cuckoofilter_table.hpp:111-136: tag j of bucket i from the packed table.

@@ -50,6 +50,9 @@ struct ProbeArgs {
   // 1: a Bloom filter's 256-bit block loads do not allocate in L1 (bitmask
   // plan, filters that cannot live in L1; set by the planner)
   uint32_t l1na;
+  // 1: the bitmask kernel tests several keys at once where the kind can
+  // (Ops::contains_n; set by the planner)
+  uint32_t together;
   // blocked cuckoo filter: log2(buckets per block), and the shift that turns
   // the block hash into the bucket hash (32: the bucket hash is key * C[0])
   uint32_t bcf_bucket_bits, bcf_hash_shift;

@@ -14,6 +14,7 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include "common.cuh"
 #include "probe.cuh"
@@ -53,7 +54,7 @@ struct CompactArgs {
 #ifdef __CUDACC__
 
 // The bitmask loop: every warp takes chunks of 128 keys (one 16-byte key
-// vector per lane), tests them with test(key) and writes the 128 flags as four
+// vector per lane), tests them with test(keys) (bit q: key q matches) and writes the 128 flags as four
 // 32-bit words of the key-ordered mask.  or_into: a later block-range pass ORs
 // its flags into the words of the earlier passes (every word is written by
 // exactly one warp per pass, and the passes are ordered on one stream).
@@ -73,8 +74,7 @@ __device__ __forceinline__ void bits_loop(const ProbeArgs& a, uint32_t* __restri
     if (v < n_vec) {
       const uint4 kv = __ldcs(keys4 + v);
       const uint32_t k[4] = {kv.x, kv.y, kv.z, kv.w};
-#pragma unroll
-      for (int q = 0; q < 4; q++) f |= (test(k[q]) ? 1u : 0u) << q;
+      f = test(k);
       const uint64_t p0 = v * 4;
       if (p0 < a.pre || p0 + 4 > a.n_phys) {
 #pragma unroll
@@ -97,10 +97,32 @@ __device__ __forceinline__ void bits_loop(const ProbeArgs& a, uint32_t* __restri
   }
 }
 
+// Ops with a test of several keys at once (contains_n).
+template <class Ops, class = void>
+struct HasContainsN : std::false_type {};
+template <class Ops>
+struct HasContainsN<Ops, std::void_t<decltype(&Ops::template contains_n<4>)>> : std::true_type {};
+
 template <class Ops, int MINB>
 __global__ void __launch_bounds__(256, MINB)
 probe_bits_kernel(const __grid_constant__ ProbeArgs a, uint32_t* __restrict__ bits, int or_into) {
-  bits_loop(a, bits, or_into, [&](uint32_t key) { return Ops::contains(a, key); });
+  bits_loop(a, bits, or_into, [&](const uint32_t (&k)[4]) {
+    if constexpr (HasContainsN<Ops>::value) {
+      if (a.together) {
+        // two keys' loads in flight fit 40 registers, four spill
+        if constexpr (MINB >= 6) {
+          const uint32_t lo[2] = {k[0], k[1]}, hi[2] = {k[2], k[3]};
+          return Ops::template contains_n<2>(a, lo) | Ops::template contains_n<2>(a, hi) << 2;
+        } else {
+          return Ops::template contains_n<4>(a, k);
+        }
+      }
+    }
+    uint32_t f = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) f |= (Ops::contains(a, k[q]) ? 1u : 0u) << q;
+    return f;
+  });
 }
 
 // Plan 4, filters that fit in shared memory: every CTA first copies the whole
@@ -120,7 +142,12 @@ probe_smem_kernel(const __grid_constant__ ProbeArgs a, uint32_t* __restrict__ bi
   const uint32_t* g32 = static_cast<const uint32_t*>(a.filter);
   for (uint32_t i = n_vec * 4 + threadIdx.x; i < filter_words32; i += blockDim.x) s32[i] = __ldg(g32 + i);
   __syncthreads();
-  bits_loop(a, bits, 0, [&](uint32_t key) { return Ops::contains_shared(s_filter, a, key); });
+  bits_loop(a, bits, 0, [&](const uint32_t (&k)[4]) {
+    uint32_t f = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) f |= (Ops::contains_shared(s_filter, a, k[q]) ? 1u : 0u) << q;
+    return f;
+  });
 }
 
 // Ordered compaction.  A tile is kWarps * ROWS * 32 mask words; warp w of the

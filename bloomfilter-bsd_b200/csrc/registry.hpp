@@ -22,8 +22,10 @@ using build_fn = cudaError_t (*)(const BuildArgs&, int grid, cudaStream_t);
 using occ_fn = int (*)();
 using probe_bits_fn = cudaError_t (*)(const ProbeArgs&, uint32_t* bits, int or_into, int grid, cudaStream_t);
 
-// Register-budget variants of probe_bits_kernel: 0 = 8 CTAs/SM (32 registers),
-// 1 = 4 CTAs/SM (64 registers, more filter loads in flight per thread).
+// Register-budget variants: probe_bits_kernel 0 = 6 CTAs/SM (40 registers; 8
+// and 32 for blocked cuckoo and classic Bloom filters), probe_pairs_kernel 0 =
+// 8 CTAs/SM (32 registers), 1 = 4 CTAs/SM (64 registers, more filter loads in
+// flight per thread).
 constexpr int kBitsVariants = 2;
 using pairs_fn = cudaError_t (*)(const PairsArgs&, int grid, cudaStream_t);
 // plan 4: bitmask probe against a shared-memory copy of a filter of words32
@@ -223,10 +225,11 @@ struct SmemLaunch {
 
 // Probe kernels of one Ops type; Pairs = false leaves the partitioned plan
 // out, Smem = false the shared-memory plan.
-template <class Ops, bool Pairs, bool Smem = false>
+// MINB0: resident CTAs per SM that variant 0 of the bitmask kernel is built for.
+template <class Ops, bool Pairs, bool Smem = false, int MINB0 = 8>
 ProbeKernels probe_entry() {
   using F = FusedLaunch<Ops>;
-  using B8 = BitsLaunch<Ops, 8>;
+  using B8 = BitsLaunch<Ops, MINB0>;
   using B4 = BitsLaunch<Ops, 4>;
   using P8 = PairsLaunch<Ops, 8>;
   using P4 = PairsLaunch<Ops, 4>;
@@ -248,7 +251,7 @@ ProbeKernels probe_entry() {
 template <typename Word, int W, int S, int Z, int K>
 BloomKernels bloom_entry() {
   using C = BloomCfg<Word, W, S, Z, K>;
-  return BloomKernels{static_cast<uint32_t>(sizeof(Word)), W, S, Z, K, probe_entry<BloomOps<C>, true, true>(),
+  return BloomKernels{static_cast<uint32_t>(sizeof(Word)), W, S, Z, K, probe_entry<BloomOps<C>, true, true, 6>(),
                       &BloomLaunch<C>::build, &BloomLaunch<C>::build_pairs, &BloomRangesLaunch<C>::run};
 }
 
@@ -275,7 +278,7 @@ struct CuckooLaunch {
 template <int T, int B>
 CuckooKernels cuckoo_entry() {
   using L = CuckooLaunch<T, B>;
-  return CuckooKernels{T, B, CuckooCfg<T, B>::kWordBucket, probe_entry<CuckooOps<CuckooCfg<T, B>>, false>(), &L::unpack, &L::insert, &L::pack,
+  return CuckooKernels{T, B, CuckooCfg<T, B>::kWordBucket, probe_entry<CuckooOps<CuckooCfg<T, B>>, false, false, 6>(), &L::unpack, &L::insert, &L::pack,
                        &L::count};
 }
 
