@@ -196,10 +196,13 @@ dtlg_status dtlg_batch_prepare(const dtlg_batch_item* items, uint32_t n_items, i
     const uint32_t block_bytes = kMenu[d.cfg].wb * kMenu[d.cfg].w;
     const uint32_t bpr = kBatchRangeBytes / block_bytes;  // blocks per range (a power of two)
     const uint32_t n_ranges = (d.addr.block_cnt + bpr - 1) / bpr;
-    if (d.n_build == 0 || n_ranges > kBatchMaxRanges) continue;
+    // (the buckets are indexed in 32 bits)
+    if (d.n_build == 0 || n_ranges > kBatchMaxRanges || d.n_build > 0xC0000000u) continue;
     d.staged = 1;
     d.n_ranges = n_ranges;
     d.range_shift = log2_u32(bpr);
+    d.hash_shift = 32 - clog2(d.addr.block_cnt) + d.range_shift;
+    if (d.hash_shift > 32) d.hash_shift = 32;  // fewer blocks than a range holds
     d.bucket_cap = static_cast<uint32_t>((static_cast<uint64_t>(d.n_build) * 5 / 4 + n_ranges - 1) / n_ranges) + 64;
     bucket_at[f] = bucket_words;
     cursor_at[f] = cursor_words;

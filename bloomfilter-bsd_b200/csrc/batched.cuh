@@ -68,6 +68,7 @@ struct BatchDesc {
   uint32_t* mask;                       // match bitmask, one bit per probe key (whole 128-word tiles)
   // staged build (staged != 0): range r holds blocks [r << range_shift, ...)
   uint32_t staged, n_ranges, range_shift, bucket_cap;
+  uint32_t hash_shift;          // POW2: range = block hash >> hash_shift (32: one range)
   uint32_t* bucket;             // n_ranges x bucket_cap keys
   unsigned int* cursor;         // per range: keys sorted in so far (zeroed)
 };
@@ -177,57 +178,93 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t* v, uint32_t n
   return total;
 }
 
+// The range of a key: under POW2 addressing the top bits of its block hash.
+template <bool MAGIC>
+__device__ __forceinline__ uint32_t batch_range_of(uint32_t key, const BatchDesc& d) {
+  const uint32_t h = key * mul_const(0);
+  if constexpr (MAGIC) return block_index_of<true>(h, d.addr) >> d.range_shift;
+  return __funnelshift_rc(h, 0u, d.hash_shift);
+}
+
 // Sorts one build tile of a staged filter into its range buckets.  The tile
 // is first ordered by range in shared memory, so that each range's run of
 // keys goes to its bucket as consecutive (coalesced) stores; one atomic per
-// (tile, range) reserves the run's place in the bucket.
-//   smem: s_cnt / s_gbase [kBatchMaxRanges] + s_keys [kBatchTile] = 32 KiB.
-template <class Cfg, bool MAGIC>
+// (tile, range) reserves the run's place in the bucket.  Bound by instruction
+// issue: tiles of valid keys (FULL) whose runs fit their buckets take no test
+// per key, and a run's destination is one word.
+//   smem: s_cnt / s_dst [kBatchMaxRanges] + s_keys [kBatchTile] = 32 KiB.
+template <class Cfg, bool MAGIC, bool FULL>
 __device__ __forceinline__ void scatter_tile(const BatchDesc& d, uint64_t k0, unsigned char* smem,
                                              uint32_t* s_warp) {
   constexpr int kRounds = kBatchTile / (kBatchThreads * 4);
   uint32_t* s_cnt = reinterpret_cast<uint32_t*>(smem);       // counts, then tile-local run starts
-  uint32_t* s_gbase = s_cnt + kBatchMaxRanges;                // bucket position of each run
-  uint32_t* s_keys = s_gbase + kBatchMaxRanges;               // the tile ordered by range
-  for (uint32_t i = threadIdx.x; i < d.n_ranges; i += kBatchThreads) s_cnt[i] = 0u;
+  uint32_t* s_dst = s_cnt + kBatchMaxRanges;                  // bucket index of sorted slot 0 for the run
+  uint32_t* s_keys = s_dst + kBatchMaxRanges;                 // the tile ordered by range
+  const uint32_t n_ranges = d.n_ranges, cap = d.bucket_cap;
+  for (uint32_t i = threadIdx.x; i < n_ranges; i += kBatchThreads) s_cnt[i] = 0u;
   __syncthreads();
   const uint4* k4 = reinterpret_cast<const uint4*>(d.build_keys + k0);
-  uint32_t key[kRounds * 4], slot[kRounds * 4];  // slot: range << 12 | rank within the tile's run
+  // the keys are read twice, for the counts and, from L1 or L2, for the
+  // placement: with their ranges and ranks they would not fit 64 registers
+  uint32_t slot[kRounds * 4];  // range << 12 | rank within the tile's run
 #pragma unroll
   for (int r = 0; r < kRounds; r++) {
     const uint64_t i0 = static_cast<uint64_t>(r) * (kBatchThreads * 4) + threadIdx.x * 4u;
     uint4 kv = make_uint4(0u, 0u, 0u, 0u);
-    if (k0 + i0 < d.n_build) kv = __ldcs(k4 + (i0 >> 2));
+    if (FULL || k0 + i0 < d.n_build) kv = k4[i0 >> 2];
     const uint32_t k[4] = {kv.x, kv.y, kv.z, kv.w};
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      key[r * 4 + q] = k[q];
       slot[r * 4 + q] = 0xffffffffu;
-      if (k0 + i0 + q < d.n_build) {
-        const uint32_t rg = block_index_of<MAGIC>(k[q] * mul_const(0), d.addr) >> d.range_shift;
+      if (FULL || k0 + i0 + q < d.n_build) {
+        const uint32_t rg = batch_range_of<MAGIC>(k[q], d);
         slot[r * 4 + q] = (rg << 12) | atomicAdd(&s_cnt[rg], 1u);
       }
     }
   }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < d.n_ranges; i += kBatchThreads) {
-    const uint32_t h = s_cnt[i];
-    s_gbase[i] = h ? atomicAdd(&d.cursor[i], h) : 0u;
+  bool over = false;
+  for (uint32_t i = threadIdx.x; i < n_ranges; i += kBatchThreads) {
+    const uint32_t c = s_cnt[i];
+    const uint32_t g = c ? atomicAdd(&d.cursor[i], c) : 0u;
+    // clamped, so that a run beyond its bucket cannot reach another one's index
+    s_dst[i] = i * cap + (g < cap ? g : cap);
+    over |= g + c > cap;
+  }
+  const bool any_over = __syncthreads_or(over);
+  const uint32_t n_valid = block_exclusive_scan(s_cnt, n_ranges, s_warp);
+  for (uint32_t i = threadIdx.x; i < n_ranges; i += kBatchThreads) s_dst[i] -= s_cnt[i];
+#pragma unroll
+  for (int r = 0; r < kRounds; r++) {
+    const uint64_t i0 = static_cast<uint64_t>(r) * (kBatchThreads * 4) + threadIdx.x * 4u;
+    uint4 kv = make_uint4(0u, 0u, 0u, 0u);
+    if (FULL || k0 + i0 < d.n_build) kv = __ldcs(k4 + (i0 >> 2));
+    const uint32_t k[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const uint32_t sl = slot[r * 4 + q];
+      if (FULL || sl != 0xffffffffu) s_keys[s_cnt[sl >> 12] + (sl & 0xfffu)] = k[q];
+    }
   }
   __syncthreads();
-  const uint32_t n_valid = block_exclusive_scan(s_cnt, d.n_ranges, s_warp);
-#pragma unroll
-  for (int j = 0; j < kRounds * 4; j++)
-    if (slot[j] != 0xffffffffu) s_keys[s_cnt[slot[j] >> 12] + (slot[j] & 0xfffu)] = key[j];
-  __syncthreads();
-  for (uint32_t sl = threadIdx.x; sl < n_valid; sl += kBatchThreads) {
-    const uint32_t kk = s_keys[sl];
-    const uint32_t rg = block_index_of<MAGIC>(kk * mul_const(0), d.addr) >> d.range_shift;
-    const uint32_t pos = s_gbase[rg] + (sl - s_cnt[rg]);
-    if (pos < d.bucket_cap) {
-      d.bucket[static_cast<uint64_t>(rg) * d.bucket_cap + pos] = kk;
-    } else {
-      BloomOps<Cfg>::insert(d.words, kk, d.addr);  // bucket full: direct path
+  uint32_t* bucket = d.bucket;
+  if (FULL && !any_over) {
+#pragma unroll 4
+    for (uint32_t j = 0; j < kBatchTile / kBatchThreads; j++) {
+      const uint32_t sl = j * kBatchThreads + threadIdx.x;
+      const uint32_t kk = s_keys[sl];
+      bucket[s_dst[batch_range_of<MAGIC>(kk, d)] + sl] = kk;
+    }
+  } else {
+    for (uint32_t sl = threadIdx.x; sl < n_valid; sl += kBatchThreads) {
+      const uint32_t kk = s_keys[sl];
+      const uint32_t rg = batch_range_of<MAGIC>(kk, d);
+      const uint32_t at = s_dst[rg] + sl;
+      if (at - rg * cap < cap) {
+        bucket[at] = kk;
+      } else {
+        BloomOps<Cfg>::insert(d.words, kk, d.addr);  // bucket full: direct path
+      }
     }
   }
 }
@@ -352,7 +389,13 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batched_kernel(const __grid_
       dispatch_cfg<Cfgs...>(d.cfg, [&](auto c) {
         using Cfg = decltype(c);
         if (d.staged) {
-          dispatch_addr(d.addr, [&](auto m) { scatter_tile<Cfg, decltype(m)::value>(d, k0, s_dyn, s_wtot); });
+          dispatch_addr(d.addr, [&](auto m) {
+            if (k0 + kBatchTile <= d.n_build) {
+              scatter_tile<Cfg, decltype(m)::value, true>(d, k0, s_dyn, s_wtot);
+            } else {
+              scatter_tile<Cfg, decltype(m)::value, false>(d, k0, s_dyn, s_wtot);
+            }
+          });
           return;
         }
         using Ops = BloomOps<Cfg>;
