@@ -293,8 +293,11 @@ int bits_variant_for(const dtlg_filter* f) {
     // / 384 at 16 KiB, 436 / 450 at 256)
     return probe_passes(f) > 1 || f->d.t == 16 || (f->d.t == 12 && f->d.m_actual <= (512ull << 13)) ? 0 : 1;
   }
-  if (!f->bk || f->d.k > 8) return 1;
   const uint64_t mib = f->d.m_actual >> 23;
+  // classic Bloom, k = 4: 1 MiB 391 / 415, 64 MiB 427 / 485; k = 8 567 / 634,
+  // 635 / 769; k = 2 340 / 332 at 8 MiB
+  if (f->qk) return f->d.k >= 4 && mib >= 1 && mib <= 100 ? 0 : 1;
+  if (!f->bk || f->d.k > 8) return 1;
   const uint32_t block = f->d.w * f->d.word_bytes, s = f->d.s, w = f->d.w;
   const bool zoned = f->d.kind == Kind::kZoned, u32 = f->d.word_bytes == 4;
   if (block == 32) return mib >= 68 && mib <= 116 ? 0 : 1;

@@ -23,7 +23,7 @@ using occ_fn = int (*)();
 using probe_bits_fn = cudaError_t (*)(const ProbeArgs&, uint32_t* bits, int or_into, int grid, cudaStream_t);
 
 // Register-budget variants: probe_bits_kernel 0 = 6 CTAs/SM (40 registers; 8
-// and 32 for blocked cuckoo and classic Bloom filters), probe_pairs_kernel 0 =
+// and 32 for blocked cuckoo filters), probe_pairs_kernel 0 =
 // 8 CTAs/SM (32 registers), 1 = 4 CTAs/SM (64 registers, more filter loads in
 // flight per thread).
 constexpr int kBitsVariants = 2;
