@@ -222,23 +222,25 @@ constexpr uint64_t kSmemMaxBytes = 192ull << 10;
 // 112 Gkeys/s; not allocating, 1-8 MiB: 128.7).
 constexpr uint64_t kL1NoAllocBytes = 256ull << 10;
 
-// Filters just beyond the single-pass limit that the bitmask plan still probes
-// faster, in its block-range passes, than the partitioned plan: layouts that
-// pick their words from the whole block (s = 1, and s = 2 of 16 u32 words), and
-// u32 of one word per block.  us for 2^27 probes, bitmask / partitioned, at
-// 168, 192 and 224 MiB: u32 w=16 s=1 k=4 1115/1282, 1222/1307, 1324/1286; s=2
-// 1115/1180, 1246/1266, 1338/1188; u32 w=1 k=4 940/1026, 1093/1039; at 168 MiB
-// s=1 of u32 w=2 to 8 and u64 w=4, 8 the bitmask plan is 5 to 10 % faster, at
-// 200 MiB 2 % slower.  The others are partitioned from 160 MiB on (at 168 MiB
-// u64 w=8 s=4 1878/1230, u32 w=16 s=8 1497/1178, u64 w=8 s=2 1645/1620, u64 w=1
-// 1229/1020, u32 w=4 1061/1033, zoned u32 w=16 z=2 1144/1093, z=4 1241/1174).
+// Filters just beyond the single-pass limit that are probed by the bitmask
+// plan in its block-range passes: layouts of 64-byte blocks whose words the
+// hash picks among four or more, smaller blocks that pick from all of their
+// words, u32 of one word per block, and zoned u32 z=2.  us for 2^27 probes,
+// bitmask (8 CTAs per SM) / partitioned, at 168, 192 and 224 MiB: u32 w=16 s=1
+// k=4 1121/1282, 1225/1307, 1331/1286; s=2 1127/1180, 1250/1266, 1346/1188;
+// u32 w=1 k=4 949/1026, 1099/1039; u64 w=8 s=2 1645/1620, 1736/1709, 1690/1614;
+// zoned u32 w=16 z=2 1144/1093, 1237/1140.  The others are partitioned from 160
+// MiB on (at 168 MiB u64 w=8 s=4 1878/1230, u32 w=16 s=8 1357/1178, u64 w=1
+// 1244/1020, u32 w=4 1061/1033, zoned u32 w=16 z=4 1241/1174).
 bool bitmask_band(const dtlg_filter* f) {
-  if (f->d.kind != Kind::kBloom) return false;
+  if (f->d.kind != Kind::kBloom && f->d.kind != Kind::kZoned) return false;
   const uint64_t fbytes = (f->d.m_actual + 7) / 8;
   if (fbytes <= (160ull << 20)) return false;
   // the limits leave room for MAGIC sizes, which round a request up
   const bool u32 = f->d.word_bytes == 4;
-  if (u32 && f->d.w == 16 && f->d.s <= 2) return fbytes <= (200ull << 20);
+  if (f->d.kind == Kind::kZoned) return u32 && f->d.z == 2 && fbytes <= (200ull << 20);
+  if (f->d.w * f->d.word_bytes == 64 && f->d.s * 4 <= f->d.w)
+    return fbytes <= (u32 && f->d.s == 1 ? 264ull << 20 : 210ull << 20);
   return f->d.s == 1 && (u32 || f->d.w > 1) && fbytes <= (180ull << 20);
 }
 
@@ -282,8 +284,8 @@ bool cuckoo_keys_together(const dtlg_filter* f) {
 //   u64 w=8 s=4          469/459 480/503 539/625     u32 w=16 z=4   375/374 378/394 502/521
 //   u32 w=16 s=1 k=4     444/442 450/432 489/498     u64 w=4 s=4    364/357 385/379 480/520
 //   u32 w=1 k=4          289/293 299/291 503/492     u64 w=16 k=16  717/611 723/659 784/761
-// (an 8-CTA, 32-register form was slower than 0 everywhere but for u64 w=8 s=2
-// beyond 64 MiB, 723 at 96, and z=4 and s=4 at 80 to 96).  Bloom layouts whose
+// (in one pass the 8-CTA, 32-register form was slower than 0 everywhere but for
+// u64 w=8 s=2 beyond 64 MiB, 723 at 96, and z=4 and s=4 at 80 to 96).  Bloom layouts whose
 // kernel 0 spills take kernel 1.
 int bits_variant_for(const dtlg_filter* f) {
   if (f->ck) {
@@ -310,17 +312,20 @@ int bits_variant_for(const dtlg_filter* f) {
 }
 
 // Register-budget variant of the bitmask / pair kernels for plan `mode`: the
-// caller's, else as above for the bitmask plan in one pass, 0 in the band
-// above and for the pair probe of Bloom filters, 1 for that of the others.
+// caller's, else as above for the bitmask plan in one pass, form 2 in the band
+// above, 0 for the pair probe of Bloom filters, 1 for that of the others.  In
+// the band (192 MiB, 2^27 probes, 8 / 6 / 4 CTAs per SM, us): u64 w=8 s=2 1736
+// / 1844 / 2014, zoned u32 w=16 z=2 1237 / 1447 / 1636, u32 w=16 s=1 1225 / 1222
+// / 1407.
 // Pair probe (2^27 probes, 512 MiB, 8 / 6 / 4 CTAs per SM, us): u64 w=8 s=8 k=8
 // 1195 / 1243 / 1294; the form of 8 keeps its lead where it spills (7 layouts,
 // all k >= 12: u64 w=8 s=8 k=16 at 512 MiB 83.0 against 79.7 Gkeys/s).
 int probe_variant(const dtlg_filter* f, int mode) {
   if (f->bits_variant >= 0 && f->bits_variant < kBitsVariants) return f->bits_variant;
   if (mode == 3) return (f->d.kind == Kind::kBloom || f->d.kind == Kind::kZoned) ? 0 : 1;
-  int v = bitmask_band(f) ? 0 : bits_variant_for(f);
-  if (v == 0 && f->bk) {
-    const occ_fn spill = f->pk->bits_local_bytes[0];
+  int v = bitmask_band(f) ? 2 : bits_variant_for(f);
+  if (v != 1 && f->bk) {
+    const occ_fn spill = f->pk->bits_local_bytes[v];
     if (spill && spill() != 0) v = 1;
   }
   return v;

@@ -27,6 +27,9 @@ using probe_bits_fn = cudaError_t (*)(const ProbeArgs&, uint32_t* bits, int or_i
 // 8 CTAs/SM (32 registers), 1 = 4 CTAs/SM (64 registers, more filter loads in
 // flight per thread).
 constexpr int kBitsVariants = 2;
+// A third form of the bitmask kernel, for the planner's block-range passes: 8
+// CTAs/SM (32 registers).
+constexpr int kBitsForms = 3;
 using pairs_fn = cudaError_t (*)(const PairsArgs&, int grid, cudaStream_t);
 // plan 4: bitmask probe against a shared-memory copy of a filter of words32
 // 32-bit words; chunks = 128-key chunks of the batch, sms = SM count
@@ -36,12 +39,12 @@ using smem_fn = cudaError_t (*)(const ProbeArgs&, uint32_t* bits, uint32_t words
 // The probe kernels every filter kind provides to the probe plans.
 struct ProbeKernels {
   probe_fn probe;                               // plan 1: fused probe + compaction
-  probe_bits_fn probe_bits[kBitsVariants];      // plan 2: match bitmask
-  occ_fn bits_blocks_per_sm[kBitsVariants];
+  probe_bits_fn probe_bits[kBitsForms];         // plan 2: match bitmask
+  occ_fn bits_blocks_per_sm[kBitsForms];
   pairs_fn probe_pairs[kBitsVariants];          // plan 3: partitioned (null: not offered)
   occ_fn pairs_blocks_per_sm[kBitsVariants];
   smem_fn probe_smem;                           // plan 4: filter in shared memory (null: not offered)
-  occ_fn bits_local_bytes[kBitsVariants];       // register spills per thread of each variant
+  occ_fn bits_local_bytes[kBitsForms];          // register spills per thread of each variant
   occ_fn pairs_local_bytes[kBitsVariants];
 };
 
@@ -226,15 +229,17 @@ struct SmemLaunch {
 // Probe kernels of one Ops type; Pairs = false leaves the partitioned plan
 // out, Smem = false the shared-memory plan.
 // MINB0: resident CTAs per SM that variant 0 of the bitmask kernel is built for.
-template <class Ops, bool Pairs, bool Smem = false, int MINB0 = 8>
+// PASSES: the same of the form for block-range passes.
+template <class Ops, bool Pairs, bool Smem = false, int MINB0 = 8, int PASSES = MINB0>
 ProbeKernels probe_entry() {
   using F = FusedLaunch<Ops>;
-  using B8 = BitsLaunch<Ops, MINB0>;
+  using B0 = BitsLaunch<Ops, MINB0>;
+  using BP = BitsLaunch<Ops, PASSES>;
   using B4 = BitsLaunch<Ops, 4>;
   using P8 = PairsLaunch<Ops, 8>;
   using P4 = PairsLaunch<Ops, 4>;
-  ProbeKernels k{&F::run, {&B8::run, &B4::run}, {&B8::occupancy, &B4::occupancy},
-                 {nullptr, nullptr}, {nullptr, nullptr}, nullptr, {&B8::local_bytes, &B4::local_bytes},
+  ProbeKernels k{&F::run, {&B0::run, &B4::run, &BP::run}, {&B0::occupancy, &B4::occupancy, &BP::occupancy},
+                 {nullptr, nullptr}, {nullptr, nullptr}, nullptr, {&B0::local_bytes, &B4::local_bytes, &BP::local_bytes},
                  {nullptr, nullptr}};
   if constexpr (Smem) k.probe_smem = &SmemLaunch<Ops>::run;
   if constexpr (Pairs) {
@@ -251,7 +256,7 @@ ProbeKernels probe_entry() {
 template <typename Word, int W, int S, int Z, int K>
 BloomKernels bloom_entry() {
   using C = BloomCfg<Word, W, S, Z, K>;
-  return BloomKernels{static_cast<uint32_t>(sizeof(Word)), W, S, Z, K, probe_entry<BloomOps<C>, true, true, 6>(),
+  return BloomKernels{static_cast<uint32_t>(sizeof(Word)), W, S, Z, K, probe_entry<BloomOps<C>, true, true, 6, 8>(),
                       &BloomLaunch<C>::build, &BloomLaunch<C>::build_pairs, &BloomRangesLaunch<C>::run};
 }
 

@@ -180,8 +180,8 @@ dtlg_status dtlg_batch_contains_gather(const dtlg_filter* f, const uint64_t* fil
  * 4 = match bitmask against a copy of the filter in every CTA's shared memory
  * (Bloom and classic Bloom filters of at most 192 KiB); a plan the filter does
  * not offer falls back to 2.  Automatic: 1 below 2^20 keys; 3 for filters
- * beyond 160 MiB, except some Bloom layouts that pick their words from the
- * whole block, up to 180 or 200 MiB; else 2.  variant selects the register
+ * beyond 160 MiB, except some Bloom layouts that pick their words by hash, up
+ * to 180 to 264 MiB; else 2.  variant selects the register
  * budget of the bitmask and pair kernels (-1 = automatic, by layout and size;
  * 0 = 32 registers at 8 CTAs/SM in the pair kernel and for blocked cuckoo
  * filters, else 40 at 6; 1 = 64 registers at 4 CTAs/SM).  Results never change.
