@@ -580,7 +580,7 @@ int block_build_plan(const dtlg_filter* f, uint64_t n) {
 
 // The range-by-range build (build_ranges.cuh) of a blocked Bloom filter from
 // n_phys keys: fills in its ranges and bucket capacity, false where another
-// plan is taken.  It reads and writes every word once and handles 110 to 250
+// plan is taken.  It updates every word once and handles 110 to 250
 // Gkeys/s whatever the filter's size, where the one-kernel build does 75 to
 // 180 in L2, by the sectors and words a key touches, and the coarse partition
 // 65 to 90 beyond.  Per-build us, other plan -> range by range:

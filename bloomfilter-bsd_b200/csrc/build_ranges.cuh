@@ -8,16 +8,20 @@
 //   1. key_scatter_kernel          sorts each tile of keys by range in shared
 //                                  memory and appends its runs to the ranges'
 //                                  buckets (4 bytes per key)
-//   2. bloom_build_ranges_kernel   one CTA per range: the range's words are
-//                                  read into shared memory, its bucket's keys
-//                                  ORed in with shared-memory atomics, the
-//                                  words written back, all coalesced
+//   2. bloom_build_ranges_kernel   one CTA per range: its bucket's keys are
+//                                  ORed into zeroed shared memory with
+//                                  shared-memory atomics, the words that have
+//                                  bits ORed into the filter with coalesced
+//                                  global atomics (a 32-byte sector each)
+//
+// The filter's words are never read and stored back, so builds may overlap
+// other inserts into the same words, as those of the other plans.
 //
 // Measured (u64 w=8 s=8 k=8): 2^27 keys into 256 MiB, 2034 us with the coarse
-// partition and global atomics, 1095 so: the scatter 496 (270 Gkeys/s; 0.67
+// partition and global atomics, 1056 so: the scatter 496 (270 Gkeys/s; 0.67
 // LSU wavefronts per key, the pipe 63 % busy, barriers and shared-memory
-// latency the rest), the range build 550 (0.92 wavefronts per key, 8 shared
-// atomics of 3.5 bank cycles per warp, and the words' read and write).
+// latency the rest), the range build the rest (8 shared atomics of 3.5 bank
+// cycles per warp and key, and the atomics on the words).
 //
 // A bucket holds its expected share of the keys and some slack; the keys of a
 // run that does not fit are ORed into the words by the scatter itself, before
@@ -244,40 +248,15 @@ struct RangeBlock {
   // index in shared memory of word i of the range
   __device__ __forceinline__ static uint32_t slot(uint32_t i) { return i ^ swizzle(i / kW); }
 
-  // The range's words between global and shared memory, all threads of the
-  // CTA, kU chunks of two words in flight per thread.
-  struct alignas(2 * sizeof(Word)) Pair {
-    Word x, y;
-  };
-  static constexpr uint32_t kU = 8;
-  __device__ __forceinline__ static void copy_in(Word* s_w, const Word* gw, uint32_t nw) {
-    const Pair* g2 = reinterpret_cast<const Pair*>(gw);
-    for (uint32_t i0 = threadIdx.x; i0 < nw / 2; i0 += kU * blockDim.x) {
-      Pair v[kU];
-#pragma unroll
-      for (uint32_t u = 0; u < kU; u++)
-        if (i0 + u * blockDim.x < nw / 2) v[u] = g2[i0 + u * blockDim.x];
-#pragma unroll
-      for (uint32_t u = 0; u < kU; u++) {
-        const uint32_t i = 2 * (i0 + u * blockDim.x);
-        if (i + 1 < nw) {
-          s_w[slot(i)] = v[u].x;
-          s_w[slot(i + 1)] = v[u].y;
-        }
-      }
-    }
-    if (threadIdx.x == 0 && (nw & 1u)) s_w[slot(nw - 1)] = gw[nw - 1];
-  }
-  __device__ __forceinline__ static void copy_out(Word* gw, const Word* s_w, uint32_t nw) {
-    Pair* g2 = reinterpret_cast<Pair*>(gw);
+  // ORs the range's words into the filter, a coalesced run of atomics per warp.
+  // Another insert into the same words may run at the same time, so they are
+  // never read and stored back.
+  __device__ __forceinline__ static void or_out(Word* gw, const Word* s_w, uint32_t nw) {
 #pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < nw / 2; i += blockDim.x) {
-      Pair v;
-      v.x = s_w[slot(2 * i)];
-      v.y = s_w[slot(2 * i + 1)];
-      g2[i] = v;
+    for (uint32_t i = threadIdx.x; i < nw; i += blockDim.x) {
+      const Word v = s_w[slot(i)];
+      if (v != 0) atomic_or_word<Word>(gw + i, v);
     }
-    if (threadIdx.x == 0 && (nw & 1u)) gw[nw - 1] = s_w[slot(nw - 1)];
   }
 
   __device__ __forceinline__ static void insert(Word* s_w, uint32_t lb, uint32_t key) {
@@ -328,7 +307,8 @@ __global__ void __launch_bounds__(1024) bloom_build_ranges_kernel(const __grid_c
       prefetch_l2(a.buckets + static_cast<uint64_t>(nx) * a.cap, ((f < a.cap ? f : a.cap) & ~3u) * 4);
     }
   }
-  R::copy_in(s_w, gw, nw);
+  for (uint32_t i = threadIdx.x; i < (Cfg::kBlockBytes << a.range_log2) / 16; i += blockDim.x)
+    reinterpret_cast<uint4*>(s_keys)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
   const uint4* bk = reinterpret_cast<const uint4*>(a.buckets + static_cast<uint64_t>(rg) * a.cap);
   constexpr uint32_t kU = 2;  // key vectors in flight per thread
@@ -348,7 +328,7 @@ __global__ void __launch_bounds__(1024) bloom_build_ranges_kernel(const __grid_c
     }
   }
   __syncthreads();
-  R::copy_out(gw, s_w, nw);
+  R::or_out(gw, s_w, nw);
 }
 
 #endif  // __CUDACC__
