@@ -648,7 +648,7 @@ cudaError_t launch_range_build(const dtlg_filter* f, uint64_t* words, const uint
   const size_t smem = kScatterTile * 4 + ra.n_ranges * 8;
   int occ = 0;
   cudaError_t e = cudaMemsetAsync(ra.fill, 0, ra.n_ranges * 4, stream);
-  if (e == cudaSuccess) e = allow_dynamic_smem(scatter, smem);
+  if (e == cudaSuccess) e = allow_dynamic_smem(scatter, kScatterTile * 4 + kBuildMaxRanges * 8);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, scatter, kScatterThreads, smem);
   if (e == cudaSuccess) {
     const uint32_t grid = std::min<uint32_t>(ra.n_tiles, static_cast<uint32_t>(ds.sms) * std::max(1, occ));

@@ -178,14 +178,14 @@ struct BloomLaunch {
   }
 };
 
-// Raises the kernel's dynamic shared-memory limit to `bytes` on the current
-// device (a few hundred ns; the limit belongs to the device's context; up to
-// 40 KiB fits the default limit of 48 beside the static shared memory).
+// Allows the kernel `bytes` of dynamic shared memory on the current device (a
+// few hundred ns; the limit belongs to the device's context).  All host threads
+// share the limit, so `bytes` is the most that any launch of the kernel asks
+// for, never this call's own size: a thread with a smaller launch would lower
+// the limit between another's call and its launch, which would then fail.
 template <class K>
 cudaError_t allow_dynamic_smem(K kernel, size_t bytes) {
-  return bytes <= (40u << 10) ? cudaSuccess
-                              : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(bytes));
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
 template <class Cfg>
@@ -193,7 +193,7 @@ struct BloomRangesLaunch {
   static cudaError_t run(const RangeArgs& a, uint32_t range_bytes, cudaStream_t s) {
     // a range of the largest size has an SM to itself, smaller ones share it
     const int threads = range_bytes == kBuildRangeBytes ? 1024 : 512;
-    cudaError_t e = allow_dynamic_smem(bloom_build_ranges_kernel<Cfg>, range_bytes);
+    cudaError_t e = allow_dynamic_smem(bloom_build_ranges_kernel<Cfg>, kBuildRangeBytes);
     if (e != cudaSuccess) return e;
     bloom_build_ranges_kernel<Cfg><<<a.n_ranges, threads, range_bytes, s>>>(a);
     return cudaGetLastError();

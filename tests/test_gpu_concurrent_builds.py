@@ -33,3 +33,35 @@ def test_inserts_from_several_streams(layout, m):
                 assert f.batch_insert(got, p)
         torch.cuda.synchronize()
         assert torch.equal(got, want)
+
+
+def test_builds_of_different_sizes_from_several_threads():
+    """Builds with different numbers and sizes of ranges (and so of shared
+    memory) at the same time, each thread with filters and a stream of its own:
+    every one succeeds and leaves the words of the one-kernel build."""
+    import threading
+    keys = keygen.build_keys_torch(1 << 23, 52)
+    sizes = [5 << 23, 1 << 25, 1 << 27, 200 << 23, 300 << 20, 130 << 23]
+    bad = []
+    torch.cuda.synchronize()
+
+    def work(t):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for i in range(6):
+                f = F.construct(F.blocked_bloomfilter_config(8, 8, 8, 8, 0, 1), sizes[(t + i) % len(sizes)])
+                got, want = f.alloc_filter_data(), f.alloc_filter_data()
+                try:
+                    assert f.batch_insert(got, keys)
+                    f.set_build_options(1)
+                    assert f.batch_insert(want, keys)
+                    if not torch.equal(got, want):
+                        bad.append((t, i, "words differ"))
+                except Exception as e:  # noqa: BLE001
+                    bad.append((t, i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(6)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[:3]
