@@ -594,6 +594,11 @@ int block_build_plan(const dtlg_filter* f, uint64_t n) {
 //   other layouts in L2 only for very many keys: 2^26 / 64 MiB u32 w=1 390 ->
 //   340, u64 w=4 s=4 634 -> 577, u64 w=8 z=4 633 -> 602, but 2^24 / 32 MiB 93
 //   -> 105, 150 -> 168, 150 -> 175.
+// A range is one CTA, so a filter of few ranges would leave most SMs idle: 128
+// of them at least (2^22 keys, u64 w=8 s=8: 16 / 64 / 256 KiB, 2 / 8 / 32
+// ranges, 142 -> 1042, 121 -> 283, 65 -> 89; 1 MiB, 128 ranges, 60 -> 43), 256
+// for the other layouts (2^26 keys: u64 w=4 s=4 256 KiB 772 -> 1920, 1 MiB 569
+// -> 644, 2 MiB 569 -> 560).
 bool range_build(const dtlg_filter* f, uint64_t n_phys, RangeArgs* a, uint32_t* range_bytes) {
   if (!f->bk || f->build_mode != 0 || n_phys < (1ull << 22) || n_phys > 0x70000000ull) return false;
   const uint64_t bytes = (f->d.m_actual + 7) / 8;
@@ -608,7 +613,7 @@ bool range_build(const dtlg_filter* f, uint64_t n_phys, RangeArgs* a, uint32_t* 
   a->range_log2 = 0;
   while ((block_bytes << a->range_log2) < rb) a->range_log2++;
   const uint64_t ranges = (f->d.addr.block_cnt + (1ull << a->range_log2) - 1) >> a->range_log2;
-  if (ranges < 2 || ranges > kBuildMaxRanges) return false;
+  if (ranges < (wide ? 128u : 256u) || ranges > kBuildMaxRanges) return false;
   a->n_ranges = static_cast<uint32_t>(ranges);
   a->range_shift = 32 - clog2(f->d.addr.block_cnt) + a->range_log2;  // POW2 only
   const uint64_t share = (n_phys << a->range_log2) / f->d.addr.block_cnt + 1;
@@ -956,6 +961,14 @@ dtlg_status dtlg_set_build_options(dtlg_filter* f, int mode) {
   if (mode < 0 || mode > 2) return DTLG_ERR_INVALID_CONFIG;
   f->build_mode = mode;
   return DTLG_OK;
+}
+
+int dtlg_build_plan(const dtlg_filter* f, uint32_t key_cnt) {
+  if (!f || key_cnt == 0) return 0;
+  RangeArgs ra{};
+  uint32_t range_bytes = 0;
+  if (range_build(f, key_cnt, &ra, &range_bytes)) return 3;
+  return f->bk || f->xk ? block_build_plan(f, key_cnt) : 1;
 }
 
 size_t dtlg_probe_workspace_size(uint32_t key_cnt) { return workspace_bytes(static_cast<uint64_t>(key_cnt) + 3); }

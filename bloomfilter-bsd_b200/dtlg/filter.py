@@ -143,6 +143,11 @@ class filter_base:  # noqa: N801 (reference name)
         2 keys grouped by L2-sized block range first (same words)."""
         check(lib().dtlg_set_build_options(self._h, int(mode)), "set_build_options")
 
+    def build_plan(self, key_cnt):
+        """The plan that batch_insert of key_cnt keys takes (1 or 2 as above,
+        3 range by range in shared memory)."""
+        return lib().dtlg_build_plan(self._h, int(key_cnt))
+
     def autotune(self, filter_data, keys, reps=5):
         """Times every probe plan on these keys and keeps the fastest for this
         filter (the reference's calibrate(), blocked_bloomfilter_tune_impl.hpp:
