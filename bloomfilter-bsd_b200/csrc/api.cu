@@ -580,10 +580,10 @@ int block_build_plan(const dtlg_filter* f, uint64_t n) {
 
 // The range-by-range build (build_ranges.cuh) of a blocked Bloom filter from
 // n_phys keys: fills in its ranges and bucket capacity, false where another
-// plan is taken.  It updates every word once and handles 110 to 250
-// Gkeys/s whatever the filter's size, where the one-kernel build does 75 to
-// 180 in L2, by the sectors and words a key touches, and the coarse partition
-// 65 to 90 beyond.  Per-build us, other plan -> range by range:
+// plan is taken.  It updates every word once and handles 80 to 250 Gkeys/s
+// whatever the filter's size, where the one-kernel build does 75 to 180 in L2,
+// by the sectors and words a key touches, and the coarse partition 65 to 90
+// beyond.  Per-build us, other plan -> range by range:
 //   beyond 80 MiB, one key per 40 bytes or more: u64 w=8 s=8 k=8 2^26 keys /
 //   128 MiB 1002 -> 508, 2^22 / 181 MiB 130 -> 107; u32 w=1 k=4 610 -> 390, 121
 //   -> 114 (at 64 bytes per key 142 -> 144, and u32 w=16 s=8 133 -> 151);
@@ -599,6 +599,10 @@ int block_build_plan(const dtlg_filter* f, uint64_t n) {
 // ranges, 142 -> 1042, 121 -> 283, 65 -> 89; 1 MiB, 128 ranges, 60 -> 43), 256
 // for the other layouts (2^26 keys: u64 w=4 s=4 256 KiB 772 -> 1920, 1 MiB 569
 // -> 644, 2 MiB 569 -> 560).
+// Repeated keys: 2^24 copies of D keys, u64 w=8 s=8, us per build, 8 MiB and 128
+// MiB: D = 1 17245 -> 281, 85268 -> 289; 1000 336 -> 230, 689 -> 259; 10 000 240
+// -> 224, 358 -> 265; 10^6 239 -> 141, 292 -> 184.  It loses where few copies of
+// few keys meet small batches: 2^22 copies of 10 000 keys 68 -> 79, 113 -> 124.
 bool range_build(const dtlg_filter* f, uint64_t n_phys, RangeArgs* a, uint32_t* range_bytes) {
   if (!f->bk || f->build_mode != 0 || n_phys < (1ull << 22) || n_phys > 0x70000000ull) return false;
   const uint64_t bytes = (f->d.m_actual + 7) / 8;
@@ -617,19 +621,23 @@ bool range_build(const dtlg_filter* f, uint64_t n_phys, RangeArgs* a, uint32_t* 
   a->n_ranges = static_cast<uint32_t>(ranges);
   a->range_shift = 32 - clog2(f->d.addr.block_cnt) + a->range_log2;  // POW2 only
   const uint64_t share = (n_phys << a->range_log2) / f->d.addr.block_cnt + 1;
-  a->cap = static_cast<uint32_t>((share + share / 32 + 512 + 3) & ~3ull);
+  // More than its share, for where keys repeat the ranges' shares differ: a
+  // quarter (10 000 keys 2^22 times in 8 MiB: 79 us, with an eighth 88), a
+  // sixteenth for large batches, whose scatter slows down as the buckets spread
+  // (2^27 keys over 2048 ranges: 515 us, with a quarter 526).
+  a->cap = static_cast<uint32_t>((share + share / (n_phys < (1ull << 25) ? 4 : 16) + 512 + 3) & ~3ull);
   *range_bytes = rb;
   return true;
 }
 
 // Enqueues the range-by-range build; cudaErrorMemoryAllocation when there is
-// no room for the buckets (4.1 bytes per key), with nothing enqueued.
+// no room for the buckets (4.3 to 5 bytes per key), with nothing enqueued.
 cudaError_t launch_range_build(const dtlg_filter* f, uint64_t* words, const uint32_t* keys_al, uint64_t n_phys,
                                uint32_t pre, RangeArgs ra, uint32_t range_bytes, const DeviceState& ds,
                                cudaStream_t stream) {
   const size_t bucket_bytes = round256(static_cast<uint64_t>(ra.n_ranges) * ra.cap * 4);
   char* ws = nullptr;
-  if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), bucket_bytes + ra.n_ranges * 4, ds.pool, stream) !=
+  if (cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), bucket_bytes + (ra.n_ranges + 1) * 4, ds.pool, stream) !=
       cudaSuccess) {
     cudaGetLastError();
     return cudaErrorMemoryAllocation;
@@ -645,14 +653,13 @@ cudaError_t launch_range_build(const dtlg_filter* f, uint64_t* words, const uint
   // one that the SM takes next comes into L2 (2^22 keys / 256 MiB 154 -> 132
   // us; smaller ranges share the SM, and the hint only cost: 161 -> 181)
   ra.prefetch = range_bytes == kBuildRangeBytes ? static_cast<uint32_t>(ds.sms) : 0u;
-  ra.word_bytes = f->d.word_bytes;
-  ra.w = f->d.w;
-  ra.sched = make_schedule(f->d.word_bytes * 8, f->d.w, f->d.s, f->d.z, f->d.k, true);
+  set_range_layout(f->d.word_bytes, f->d.w,
+                   make_schedule(f->d.word_bytes * 8, f->d.w, f->d.s, f->d.z, f->d.k, true), &ra);
   ra.n_tiles = static_cast<uint32_t>((n_phys + kScatterTile - 1) / kScatterTile);
   const auto scatter = ra.addr.magic_mode ? key_scatter_kernel<true> : key_scatter_kernel<false>;
   const size_t smem = kScatterTile * 4 + ra.n_ranges * 8;
   int occ = 0;
-  cudaError_t e = cudaMemsetAsync(ra.fill, 0, ra.n_ranges * 4, stream);
+  cudaError_t e = cudaMemsetAsync(ra.fill, 0, (ra.n_ranges + 1) * 4, stream);
   if (e == cudaSuccess) e = allow_dynamic_smem(scatter, kScatterTile * 4 + kBuildMaxRanges * 8);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, scatter, kScatterThreads, smem);
   if (e == cudaSuccess) {

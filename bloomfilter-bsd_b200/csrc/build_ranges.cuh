@@ -18,14 +18,14 @@
 // other inserts into the same words, as those of the other plans.
 //
 // Measured (u64 w=8 s=8 k=8): 2^27 keys into 256 MiB, 2034 us with the coarse
-// partition and global atomics, 1056 so: the scatter 496 (270 Gkeys/s; 0.67
-// LSU wavefronts per key, the pipe 63 % busy, barriers and shared-memory
-// latency the rest), the range build the rest (8 shared atomics of 3.5 bank
-// cycles per warp and key, and the atomics on the words).
+// partition and global atomics, 1042 so: the scatter 515 (260 Gkeys/s; 0.67
+// LSU wavefronts per key, the pipe some 60 % busy, barriers and shared-memory
+// latency the rest), the range build 527 (8 shared atomics of 3.5 bank cycles
+// per warp and key, and the atomics on the words).
 //
 // A bucket holds its expected share of the keys and some slack; the keys of a
-// run that does not fit are ORed into the words by the scatter itself, before
-// the second kernel reads them, so any key distribution gives the same words.
+// run that does not fit are ORed into the words by the scatter itself, so any
+// key distribution gives the same words.
 #pragma once
 
 #include <cstdint>
@@ -41,6 +41,14 @@ constexpr int kScatterThreads = 1024;
 constexpr int kScatterKeysPerThread = 16;
 constexpr uint32_t kScatterTile = kScatterThreads * kScatterKeysPerThread;
 
+// One draw of a layout known at run time: (key * mul >> shift) & (2^bits - 1),
+// then `first` (word or bit) is added.
+struct RangeDraw {
+  uint32_t mul;     // 0: the constant hash 0
+  uint32_t fields;  // shift | bits << 8 | first << 16
+};
+constexpr uint32_t kMaxDraws = 32;  // a word draw for each of 16 groups, 16 bit draws at most
+
 struct RangeArgs {
   const uint32_t* keys_al;  // 16-byte aligned key base (see ProbeArgs)
   uint64_t n_phys;
@@ -52,37 +60,37 @@ struct RangeArgs {
   uint32_t n_tiles;
   uint32_t cap;             // keys per bucket, a multiple of 4; n_ranges * cap < 2^32
   uint32_t* buckets;        // n_ranges x cap
-  unsigned int* fill;       // per range: keys sent to its bucket, may exceed cap (zeroed)
+  unsigned int* fill;       // per range: keys sent to its bucket, may exceed cap; last: 1 when one did (zeroed)
   uint32_t prefetch;        // the range build hints its range + prefetch into L2 (0: none)
   void* filter;
-  // the layout, for the keys that find their bucket full
-  uint32_t word_bytes, w;
-  Schedule sched;
+  // the layout, for the keys that find their bucket full: per group its word
+  // draw, then its `nbit` bit draws (every group has as many)
+  uint32_t word_bytes, w, ng, nbit;
+  RangeDraw draw[kMaxDraws];
 };
+
+// The layout fields of `a` from a schedule.
+inline void set_range_layout(uint32_t word_bytes, uint32_t w, const Schedule& sched, RangeArgs* a) {
+  a->word_bytes = word_bytes;
+  a->w = w;
+  a->ng = sched.ng;
+  a->nbit = sched.g[0].nbit;
+  RangeDraw* out = a->draw;
+  for (uint32_t g = 0; g < sched.ng; g++) {
+    const Group& gr = sched.g[g];
+    *out++ = {gr.wbits ? mul_const(gr.wsel) : 0u, static_cast<uint32_t>(gr.wshift | gr.wbits << 8 | gr.wconst << 16)};
+    for (uint32_t j = 0; j < gr.nbit; j++) {
+      const BitDraw& d = gr.bit[j];
+      *out++ = {d.sel == kSelZero ? 0u : mul_const(d.sel), static_cast<uint32_t>(d.shift | d.bits << 8 | d.off << 16)};
+    }
+  }
+}
 
 #ifdef __CUDACC__
 
 // Hints `bytes` (a multiple of 16) from a 16-byte aligned address into L2.
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(bytes) : "memory");
-}
-
-// BloomOps::insert for a layout known at run time, one 32-bit atomic per bit.
-static __device__ __noinline__ void insert_any(const RangeArgs& a, uint32_t key) {
-  const uint32_t per = a.word_bytes / 4;
-  unsigned int* base = static_cast<unsigned int*>(a.filter) +
-                       static_cast<uint64_t>(block_index(key * mul_const(0), a.addr)) * a.w * per;
-  for (uint32_t g = 0; g < a.sched.ng; g++) {
-    const Group& gr = a.sched.g[g];
-    auto draw = [&](uint32_t sel, uint32_t shift, uint32_t bits) {
-      return sel == kSelZero ? 0u : (key * mul_const(static_cast<int>(sel)) >> shift) & ((1u << bits) - 1u);
-    };
-    const uint32_t word = gr.wconst + (gr.wbits ? draw(gr.wsel, gr.wshift, gr.wbits) : 0u);
-    for (uint32_t j = 0; j < gr.nbit; j++) {
-      const uint32_t b = draw(gr.bit[j].sel, gr.bit[j].shift, gr.bit[j].bits) + gr.bit[j].off;
-      atomicOr(base + word * per + (b >> 5), 1u << (b & 31u));
-    }
-  }
 }
 
 // The range of a key: the top bits of its block hash under POW2 addressing.
@@ -93,8 +101,114 @@ __device__ __forceinline__ uint32_t build_range_of(uint32_t key, const RangeArgs
   return h >> a.range_shift;
 }
 
+// What the checked write-out reads, copied from the kernel's parameters, whose
+// fields would be loaded from memory again after every atomic.
+struct OverflowArgs {
+  Addr addr;
+  uint32_t range_sel, cap, word_bytes, w, ng, nbit;  // range_sel: range_log2 (MAGIC) or range_shift
+  uint32_t* buckets;
+  void* filter;
+};
+
+// Inserts the keys of the lanes with `over` set straight into the words, whole
+// warps only.  The word groups of a key go to neighbouring lanes, one atomic
+// each and one request per 32-byte sector (as BloomOps::insert_lanes).  Buckets
+// overflow where keys repeat: where lanes have their neighbour's key, the
+// copies within the warp are inserted once, and bits that are set already (a
+// load from L1, which may miss newer ones) take no atomic.
+// stage: 32 words of shared memory of this warp's own.
+template <bool MAGIC>
+__device__ __forceinline__ void insert_overflow(const OverflowArgs& a, uint32_t key, bool over, uint32_t* stage,
+                                                const RangeDraw* s_draw) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t todo = __ballot_sync(0xffffffffu, over);
+  if (todo == 0) return;
+  const bool same = __shfl_xor_sync(0xffffffffu, key, 1) == key;
+  if (__popc(__ballot_sync(0xffffffffu, over && same)) >= 3) {
+    bool first = false;
+    if (over) first = lane == static_cast<uint32_t>(__ffs(__match_any_sync(todo, key)) - 1);
+    todo = __ballot_sync(0xffffffffu, first);
+  }
+  if (todo >> lane & 1u) stage[__popc(todo & ((1u << lane) - 1u))] = key;
+  __syncwarp();
+  const uint32_t per = 32u / a.ng;  // keys per step
+  const uint32_t n = __popc(todo);
+  const RangeDraw* d = s_draw + (lane % a.ng) * (1 + a.nbit);
+  struct Draw {
+    uint32_t mul, shift, mask, first;
+    __device__ __forceinline__ Draw(const RangeDraw& r)
+        : mul(r.mul), shift(r.fields & 0xffu), mask((1u << (r.fields >> 8 & 0xffu)) - 1u), first(r.fields >> 16) {}
+    __device__ __forceinline__ uint32_t of(uint32_t k) const { return (k * mul >> shift & mask) + first; }
+  };
+  const Draw word(d[0]), bit(d[1]);
+  const uint32_t halves = a.word_bytes / 4;  // 32-bit words per word
+  unsigned int* const base = static_cast<unsigned int*>(a.filter);
+  for (uint32_t i = lane < per * a.ng ? lane / a.ng : n; i < n; i += per) {
+    const uint32_t k = stage[i];
+    const uint32_t blk = block_index_of<MAGIC>(k * mul_const(0), a.addr);
+    unsigned int* p = base + static_cast<uint64_t>(blk) * (a.w * halves) + word.of(k) * halves;
+    uint32_t b = bit.of(k);
+    if (a.nbit == 1) {
+      p += b >> 5;
+      const uint32_t m = 1u << (b & 31u);
+      if ((ld_weak_32(p) & m) == 0) atomicOr(p, m);
+    } else {
+      unsigned long long m = 1ull << b;
+      for (uint32_t j = 2; j <= a.nbit; j++) m |= 1ull << Draw(d[j]).of(k);
+      if (halves == 2) {
+        unsigned long long* p2 = reinterpret_cast<unsigned long long*>(p);
+        if ((ld_weak_64(p2) & m) != m) atomicOr(p2, m);
+      } else if ((ld_weak_32(p) & m) != m) {
+        atomicOr(p, static_cast<unsigned int>(m));
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// Writes a tile's n sorted keys to their buckets, those that do not fit into
+// the words.  A function of its own, all threads of the CTA: its registers
+// would spill the tile loop's.
+template <bool MAGIC>
+__device__ __noinline__ void write_tile_checked(const RangeArgs& args, uint32_t n, uint32_t* s_keys) {
+  __shared__ RangeDraw s_draw[kMaxDraws];
+  if (threadIdx.x < kMaxDraws) s_draw[threadIdx.x] = args.draw[threadIdx.x];
+  __syncthreads();
+  const uint32_t* s_dst = s_keys + kScatterTile + args.n_ranges;
+  const OverflowArgs a{args.addr, MAGIC ? args.range_log2 : args.range_shift, args.cap, args.word_bytes, args.w, args.ng,
+                       args.nbit, args.buckets, args.filter};
+  auto place = [&](uint32_t sl, uint32_t* key, uint32_t* at) {  // does sorted slot sl's key fit its bucket
+    *key = s_keys[sl];
+    const uint32_t h = *key * mul_const(0);
+    const uint32_t r = (MAGIC ? block_index_of<true>(h, a.addr) : h) >> a.range_sel;
+    *at = s_dst[r] + sl;
+    return *at - r * a.cap < a.cap;
+  };
+  uint32_t over_steps = 0;  // steps in which a key of this warp does not fit
+#pragma unroll 4
+  for (uint32_t j = 0; j < kScatterKeysPerThread; j++) {
+    const uint32_t sl = j * kScatterThreads + threadIdx.x;
+    bool over = false;
+    if (sl < n) {
+      uint32_t key, at;
+      over = !place(sl, &key, &at);
+      if (!over) a.buckets[at] = key;
+    }
+    if (__any_sync(0xffffffffu, over)) over_steps |= 1u << j;
+  }
+  if (over_steps != 0) args.fill[args.n_ranges] = 1;  // tells the range build that keys repeat
+  for (; over_steps != 0; over_steps &= over_steps - 1) {
+    const uint32_t sl = (__ffs(over_steps) - 1) * kScatterThreads + threadIdx.x;
+    uint32_t key = 0, at;
+    const bool over = sl < n && !place(sl, &key, &at);
+    __syncwarp();  // the keys are read: their slots are the warp's stage
+    insert_overflow<MAGIC>(a, key, over, s_keys + (sl & ~31u), s_draw);
+  }
+}
+
 // Shared memory of a scatter CTA (dynamic): the tile's keys sorted by range,
-// the ranges' counts (then run starts), the ranges' destinations.
+// the ranges' counts (then run starts), the ranges' destinations (write_tile_checked
+// finds them there).
 struct KeyScatter {
   static constexpr uint32_t THREADS = kScatterThreads, kTile = kScatterTile;
   static constexpr int kVecs = kScatterKeysPerThread / 4;
@@ -189,16 +303,7 @@ struct KeyScatter {
         a.buckets[s_dst[build_range_of<MAGIC>(key, a)] + sl] = key;
       }
     } else {
-      for (uint32_t sl = threadIdx.x; sl < hi - lo; sl += THREADS) {
-        const uint32_t key = s_keys[sl];
-        const uint32_t r = build_range_of<MAGIC>(key, a);
-        const uint32_t at = s_dst[r] + sl;
-        if (at - r * a.cap < a.cap) {
-          a.buckets[at] = key;
-        } else {
-          insert_any(a, key);
-        }
-      }
+      write_tile_checked<MAGIC>(a, hi - lo, s_keys);
     }
     __syncthreads();
   }
@@ -242,6 +347,12 @@ struct RangeBlock {
   using Word = typename Cfg::word_t;
   using Ops = BloomOps<Cfg>;
   static constexpr uint32_t kW = Cfg::kW;
+  static constexpr bool fits_draws() {
+    for (uint32_t g = 0; g < Ops::kS.ng; g++)
+      if (Ops::kS.g[g].nbit != Ops::kS.g[0].nbit) return false;
+    return Ops::kS.ng * (1 + Ops::kS.g[0].nbit) <= kMaxDraws;
+  }
+  static_assert(fits_draws(), "RangeArgs::draw holds every layout");
   static constexpr uint32_t kRowShift = Cfg::kBlockBytes < 128 ? clog2(128 / Cfg::kBlockBytes) : 0;
 
   __device__ __forceinline__ static uint32_t swizzle(uint32_t lb) { return (lb >> kRowShift) & (kW - 1); }
@@ -259,7 +370,12 @@ struct RangeBlock {
     }
   }
 
+  // TEST: bits that are set already take no atomic.
+  template <bool TEST>
   __device__ __forceinline__ static void insert(Word* s_w, uint32_t lb, uint32_t key) {
+    auto set = [](uint32_t* p, uint32_t m) {
+      if (!TEST || (*static_cast<volatile uint32_t*>(p) & m) != m) atomicOr(p, m);
+    };
     const uint32_t swz = swizzle(lb);
     Word* base = s_w + lb * kW;
     static_for<Ops::kS.ng>([&](auto G) {
@@ -270,15 +386,15 @@ struct RangeBlock {
         // one bit: one 32-bit atomic on the half that holds it
         constexpr BitDraw b = grp.bit[0];
         const uint32_t bit = ((hash_sel<b.sel>(key) >> b.shift) & ((1u << b.bits) - 1u)) + b.off;
-        atomicOr(p + (bit >> 5), 1u << (bit & 31u));
+        set(p + (bit >> 5), 1u << (bit & 31u));
       } else if constexpr (sizeof(Word) == 8) {
         // 32-bit atomics: 64-bit shared-memory ORs are slower
         const unsigned long long m = Ops::template group_mask<g>(key);
         const uint32_t lo = static_cast<uint32_t>(m), hi = static_cast<uint32_t>(m >> 32);
-        if (lo) atomicOr(p, lo);
-        if (hi) atomicOr(p + 1, hi);
+        if (lo) set(p, lo);
+        if (hi) set(p + 1, hi);
       } else {
-        atomicOr(p, static_cast<uint32_t>(Ops::template group_mask<g>(key)));
+        set(p, static_cast<uint32_t>(Ops::template group_mask<g>(key)));
       }
     });
   }
@@ -290,10 +406,11 @@ __global__ void __launch_bounds__(1024) bloom_build_ranges_kernel(const __grid_c
   using Word = typename Cfg::word_t;
   extern __shared__ __align__(16) uint32_t s_keys[];
   Word* s_w = reinterpret_cast<Word*>(s_keys);
-  const uint32_t rg = blockIdx.x;
+  const uint32_t rg = blockIdx.x, lane = threadIdx.x & 31u;
   const uint32_t fill = a.fill[rg];
   const uint32_t cnt = fill < a.cap ? fill : a.cap;
   if (cnt == 0) return;
+  const bool repeats = a.fill[a.n_ranges] != 0;
   const uint32_t blk0 = rg << a.range_log2;
   const uint32_t left = a.addr.block_cnt - blk0;
   const uint32_t nw = (left < (1u << a.range_log2) ? left : 1u << a.range_log2) * Cfg::kW;
@@ -312,18 +429,39 @@ __global__ void __launch_bounds__(1024) bloom_build_ranges_kernel(const __grid_c
   __syncthreads();
   const uint4* bk = reinterpret_cast<const uint4*>(a.buckets + static_cast<uint64_t>(rg) * a.cap);
   constexpr uint32_t kU = 2;  // key vectors in flight per thread
-  for (uint32_t v0 = threadIdx.x; v0 * 4 < cnt; v0 += kU * blockDim.x) {
+  for (uint32_t v0 = threadIdx.x & ~31u; v0 * 4 < cnt; v0 += kU * blockDim.x) {
+    const uint32_t v = v0 + lane;
     uint4 kv[kU];
 #pragma unroll
     for (uint32_t u = 0; u < kU; u++)
-      kv[u] = (v0 + u * blockDim.x) * 4 < cnt ? __ldcs(bk + v0 + u * blockDim.x) : make_uint4(0, 0, 0, 0);
+      kv[u] = (v + u * blockDim.x) * 4 < cnt ? __ldcs(bk + v + u * blockDim.x) : make_uint4(0, 0, 0, 0);
+    // Atomics on the same words wait for one another, loads do not: where
+    // neighbours are often equal (copies of some 60 keys or fewer), bits are
+    // tested first.
+    bool same = false;
+    if (repeats) {
+#pragma unroll
+      for (uint32_t u = 0; u < kU; u++) same |= kv[u].x == kv[u].y || kv[u].y == kv[u].z || kv[u].z == kv[u].w;
+    }
+    if (repeats && __popc(__ballot_sync(0xffffffffu, same && (v + blockDim.x) * 4 + 3 < cnt)) >= 3) {
+      const uint32_t* b32 = reinterpret_cast<const uint32_t*>(bk);
+#pragma unroll 4
+      for (uint32_t j = 0; j < kU * 4; j++) {
+        const uint32_t i = (v + j / 4 * blockDim.x) * 4 + j % 4;
+        if (i < cnt) {
+          const uint32_t key = __ldg(b32 + i);
+          R::template insert<true>(s_w, block_index(key * mul_const(0), a.addr) - blk0, key);
+        }
+      }
+      continue;
+    }
 #pragma unroll
     for (uint32_t u = 0; u < kU; u++) {
       const uint32_t k[4] = {kv[u].x, kv[u].y, kv[u].z, kv[u].w};
 #pragma unroll
       for (uint32_t q = 0; q < 4; q++) {
-        if ((v0 + u * blockDim.x) * 4 + q < cnt)
-          R::insert(s_w, block_index(k[q] * mul_const(0), a.addr) - blk0, k[q]);
+        if ((v + u * blockDim.x) * 4 + q < cnt)
+          R::template insert<false>(s_w, block_index(k[q] * mul_const(0), a.addr) - blk0, k[q]);
       }
     }
   }
