@@ -594,11 +594,11 @@ int block_build_plan(const dtlg_filter* f, uint64_t n) {
 //   other layouts in L2 only for very many keys: 2^26 / 64 MiB u32 w=1 390 ->
 //   340, u64 w=4 s=4 634 -> 577, u64 w=8 z=4 633 -> 602, but 2^24 / 32 MiB 93
 //   -> 105, 150 -> 168, 150 -> 175.
-// A range is one CTA, so a filter of few ranges would leave most SMs idle: 128
-// of them at least (2^22 keys, u64 w=8 s=8: 16 / 64 / 256 KiB, 2 / 8 / 32
-// ranges, 142 -> 1042, 121 -> 283, 65 -> 89; 1 MiB, 128 ranges, 60 -> 43), 256
-// for the other layouts (2^26 keys: u64 w=4 s=4 256 KiB 772 -> 1920, 1 MiB 569
-// -> 644, 2 MiB 569 -> 560).
+// A range is one CTA, so a filter of few ranges would leave most SMs idle: 64 of
+// them at least (u64 w=8 s=8, one-kernel build -> range by range: 256 KiB, 32
+// ranges, 2^22 keys 65 -> 89, 2^26 967 -> 1237; 512 KiB, 64 ranges, 68 -> 68,
+// 925 -> 731), 256 for the other layouts (2^26 keys: u64 w=4 s=4 256 KiB 772 ->
+// 1920, 1 MiB 569 -> 644, 2 MiB 569 -> 560).
 // Repeated keys: 2^24 copies of D keys, u64 w=8 s=8, us per build, 8 MiB and 128
 // MiB: D = 1 17245 -> 281, 85268 -> 289; 1000 336 -> 230, 689 -> 259; 10 000 240
 // -> 224, 358 -> 265; 10^6 239 -> 141, 292 -> 184.  It loses where few copies of
@@ -617,7 +617,7 @@ bool range_build(const dtlg_filter* f, uint64_t n_phys, RangeArgs* a, uint32_t* 
   a->range_log2 = 0;
   while ((block_bytes << a->range_log2) < rb) a->range_log2++;
   const uint64_t ranges = (f->d.addr.block_cnt + (1ull << a->range_log2) - 1) >> a->range_log2;
-  if (ranges < (wide ? 128u : 256u) || ranges > kBuildMaxRanges) return false;
+  if (ranges < (wide ? 64u : 256u) || ranges > kBuildMaxRanges) return false;
   a->n_ranges = static_cast<uint32_t>(ranges);
   a->range_shift = 32 - clog2(f->d.addr.block_cnt) + a->range_log2;  // POW2 only
   const uint64_t share = (n_phys << a->range_log2) / f->d.addr.block_cnt + 1;

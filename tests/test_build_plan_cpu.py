@@ -21,7 +21,7 @@ def test_few_ranges_keep_the_one_kernel_build(layout):
 
 
 @pytest.mark.parametrize("layout,kib,n,plan", [
-    ((8, 8, 8, 1, 8), 1024, 1 << 22, 3), ((8, 8, 8, 1, 8), 8192, 1 << 22, 3),
+    ((8, 8, 8, 1, 8), 512, 1 << 22, 3), ((8, 8, 8, 1, 8), 8192, 1 << 22, 3),
     ((8, 8, 8, 1, 8), 8192, (1 << 22) - 1, 1), ((8, 8, 8, 1, 8), 64 << 10, 1 << 22, 1),
     ((8, 8, 8, 1, 8), 64 << 10, 1 << 23, 3), ((8, 8, 8, 1, 8), 128 << 10, 1 << 22, 3),
     ((8, 8, 8, 1, 8), 256 << 10, 1 << 22, 2), ((8, 8, 8, 1, 8), 512 << 10, 1 << 28, 3),
