@@ -13,7 +13,6 @@
 
 #include <cstdint>
 #include <mutex>
-#include <vector>
 
 namespace dtlg {
 
@@ -27,59 +26,69 @@ struct ResultSlot {
 
 // The slots of one device: a call takes one and gives it back, so threads and
 // streams never share one.  At most kMax exist; a call that finds none left
-// (or cannot make one) goes without.
+// (or cannot make one) goes without.  The bookkeeping has a fixed size, so that
+// nothing here throws: the callers are C entry points.
 class ResultSlots {
  public:
   static constexpr int kMax = 16;
 
-  ResultSlot* acquire(size_t dev_bytes) {
+  ResultSlot* acquire(size_t dev_bytes) noexcept {
+    ResultSlot* s = nullptr;
     {
       std::lock_guard<std::mutex> lk(mu_);
-      if (!free_.empty()) {
-        ResultSlot* s = free_.back();
-        free_.pop_back();
-        return s;
+      if (n_free_ != 0) return free_[--n_free_];
+      for (int i = 0; i < kMax && !s; i++) {
+        if (!made_[i]) {
+          made_[i] = true;
+          s = &slots_[i];
+        }
       }
-      if (made_ == kMax) return nullptr;
-      made_++;
     }
-    // allocations are no part of a capture that another thread may have open
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    ResultSlot* s = new ResultSlot();
+    if (!s) return nullptr;
+    RelaxedCapture relaxed;
+    *s = ResultSlot{};
     cudaError_t e = cudaMalloc(&s->dev, dev_bytes);
     if (e == cudaSuccess)
       e = cudaHostAlloc(reinterpret_cast<void**>(&s->host), 64, cudaHostAllocMapped | cudaHostAllocPortable);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&s->host_dev), s->host, 0);
-    if (e == cudaSuccess) s->host[0] = 0;
-    cudaThreadExchangeStreamCaptureMode(&mode);
     if (e != cudaSuccess) {
       cudaGetLastError();
       drop(s);
       return nullptr;
     }
+    s->host[0] = 0;
     return s;
   }
 
-  void release(ResultSlot* s) {
+  void release(ResultSlot* s) noexcept {
     std::lock_guard<std::mutex> lk(mu_);
-    free_.push_back(s);
+    free_[n_free_++] = s;
   }
 
   // A slot whose call failed: its kernel may never have run, or still run, so
   // it is not used again (freeing waits for the device).
-  void drop(ResultSlot* s) {
+  void drop(ResultSlot* s) noexcept {
+    RelaxedCapture relaxed;
     if (s->dev) cudaFree(s->dev);
     if (s->host) cudaFreeHost(s->host);
-    delete s;
     std::lock_guard<std::mutex> lk(mu_);
-    made_--;
+    made_[s - slots_] = false;
   }
 
  private:
+  // Allocating and freeing are no part of a capture that another thread may
+  // have open, and would end it in the default mode.
+  struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  };
+
   std::mutex mu_;
-  std::vector<ResultSlot*> free_;
-  int made_ = 0;
+  ResultSlot slots_[kMax];
+  bool made_[kMax] = {};
+  ResultSlot* free_[kMax] = {};
+  int n_free_ = 0;
 };
 
 }  // namespace dtlg
