@@ -320,8 +320,11 @@ int bits_variant_for(const dtlg_filter* f) {
 // Pair probe (2^27 probes, 512 MiB, 8 / 6 / 4 CTAs per SM, us): u64 w=8 s=8 k=8
 // 1195 / 1243 / 1294; the form of 8 keeps its lead where it spills (7 layouts,
 // all k >= 12: u64 w=8 s=8 k=16 at 512 MiB 83.0 against 79.7 Gkeys/s).
+// The caller's 0 is form 2 where the bitmask plan takes several passes, so that
+// the tuner reaches what the planner takes in the band.
 int probe_variant(const dtlg_filter* f, int mode) {
-  if (f->bits_variant >= 0 && f->bits_variant < kBitsVariants) return f->bits_variant;
+  if (f->bits_variant >= 0 && f->bits_variant < kBitsVariants)
+    return mode == 2 && f->bits_variant == 0 && probe_passes(f) > 1 ? 2 : f->bits_variant;
   if (mode == 3) return (f->d.kind == Kind::kBloom || f->d.kind == Kind::kZoned) ? 0 : 1;
   int v = bitmask_band(f) ? 2 : bits_variant_for(f);
   if (v != 1 && f->bk) {

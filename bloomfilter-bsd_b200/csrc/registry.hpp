@@ -27,8 +27,8 @@ using probe_bits_fn = cudaError_t (*)(const ProbeArgs&, uint32_t* bits, int or_i
 // 8 CTAs/SM (32 registers), 1 = 4 CTAs/SM (64 registers, more filter loads in
 // flight per thread).
 constexpr int kBitsVariants = 2;
-// A third form of the bitmask kernel, for the planner's block-range passes: 8
-// CTAs/SM (32 registers).
+// A third form of the bitmask kernel, variant 0 of Bloom filters probed in
+// block-range passes: 8 CTAs/SM (32 registers).
 constexpr int kBitsForms = 3;
 using pairs_fn = cudaError_t (*)(const PairsArgs&, int grid, cudaStream_t);
 // plan 4: bitmask probe against a shared-memory copy of a filter of words32

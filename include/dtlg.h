@@ -183,8 +183,9 @@ dtlg_status dtlg_batch_contains_gather(const dtlg_filter* f, const uint64_t* fil
  * beyond 160 MiB, except some Bloom layouts that pick their words by hash, up
  * to 180 to 264 MiB; else 2.  variant selects the register
  * budget of the bitmask and pair kernels (-1 = automatic, by layout and size;
- * 0 = 32 registers at 8 CTAs/SM in the pair kernel and for blocked cuckoo
- * filters, else 40 at 6; 1 = 64 registers at 4 CTAs/SM).  Results never change.
+ * 0 = 32 registers at 8 CTAs/SM in the pair kernel, for Bloom filters probed in
+ * several block-range passes and for blocked cuckoo filters, else 40 at 6; 1 =
+ * 64 registers at 4 CTAs/SM).  Results never change.
  * (The reference's counterpart is its per-config SIMD unroll factor,
  * blocked_bloomfilter_tune.hpp:21-56.) */
 dtlg_status dtlg_set_probe_options(dtlg_filter* f, int mode, int variant);
