@@ -225,13 +225,23 @@ constexpr uint64_t kL1NoAllocBytes = 256ull << 10;
 // Filters just beyond the single-pass limit that are probed by the bitmask
 // plan in its block-range passes: layouts of 64-byte blocks whose words the
 // hash picks among four or more, smaller blocks that pick from all of their
-// words, u32 of one word per block, and zoned u32 z=2.  us for 2^27 probes,
-// bitmask (8 CTAs per SM) / partitioned, at 168, 192 and 224 MiB: u32 w=16 s=1
-// k=4 1121/1282, 1225/1307, 1331/1286; s=2 1127/1180, 1250/1266, 1346/1188;
-// u32 w=1 k=4 949/1026, 1099/1039; u64 w=8 s=2 1645/1620, 1736/1709, 1690/1614;
-// zoned u32 w=16 z=2 1144/1093, 1237/1140.  The others are partitioned from 160
-// MiB on (at 168 MiB u64 w=8 s=4 1878/1230, u32 w=16 s=8 1357/1178, u64 w=1
-// 1244/1020, u32 w=4 1061/1033, zoned u32 w=16 z=4 1241/1174).
+// words, u32 of one or two words per block, and zoned u32 z=2.  us for 2^26
+// probes, bitmask (8 CTAs per SM) / partitioned:
+//   MiB                 168      184      200      208      224      256
+//   u32 w=16 s=1 k=4    581/661  611/666  644/671  660/673  682/667  741/649
+//   u32 w=16 s=2 k=4    584/611  619/628  650/628  671/642
+//   u64 w=8 s=1 k=4     607/669  632/674  661/678  675/682  690/675
+//   u64 w=8 s=2         843/832  864/845  870/847  880/859  861/836
+//   zoned u32 w=16 z=2  587/569  625/591  654/593
+//   u32 w=1 k=4         494/534  544/538  590/539      (176: 518/539)
+//   u32 w=2 s=2 k=8     516/532  554/533               (176: 534/532)
+//   u32 w=2, w=4 s=1    556/601  583/604  615/601
+//   u64 w=2 s=1 k=4     582/618  601/616  626/616
+// u64 w=8 s=2, zoned u32 and the largest u32 w=16 s=1 filters would be 1 to 14 %
+// faster partitioned; they stay here, as the ABI tests have it, with an eighth of
+// a byte of workspace per key instead of 8.3.  The others are partitioned from 160
+// MiB on (at 168 MiB, 2^27 probes: u64 w=8 s=4 1878/1230, u32 w=16 s=8 1357/1178,
+// u64 w=1 1244/1020, zoned u32 w=16 z=4 1241/1174; 2^26: u32 w=4 s=4 546/534).
 bool bitmask_band(const dtlg_filter* f) {
   if (f->d.kind != Kind::kBloom && f->d.kind != Kind::kZoned) return false;
   const uint64_t fbytes = (f->d.m_actual + 7) / 8;
@@ -241,7 +251,8 @@ bool bitmask_band(const dtlg_filter* f) {
   if (f->d.kind == Kind::kZoned) return u32 && f->d.z == 2 && fbytes <= (200ull << 20);
   if (f->d.w * f->d.word_bytes == 64 && f->d.s * 4 <= f->d.w)
     return fbytes <= (u32 && f->d.s == 1 ? 264ull << 20 : 210ull << 20);
-  return f->d.s == 1 && (u32 || f->d.w > 1) && fbytes <= (180ull << 20);
+  if (f->d.s == 1 && f->d.w > 1) return fbytes <= (194ull << 20);
+  return u32 && f->d.w <= 2 && f->d.s == f->d.w && fbytes <= (f->d.w == 1 ? 182ull << 20 : 176ull << 20);
 }
 
 int probe_plan(const dtlg_filter* f, uint64_t n) {
@@ -263,15 +274,35 @@ int probe_plan(const dtlg_filter* f, uint64_t n) {
   return mode;
 }
 
-// Cuckoo tables that hit L1 on part of the loads only are probed key by key:
-// with more loads in flight the lines are gone before they are used again.  us
-// for 2^26 probes, key by key / together, at 64, 256, 320, 512 and 1024 KiB:
-// t=8 280/274 315/336 381/421 458/466 510/473, t=32 245/268 353/361 398/415
-// 458/463 508/510, t=16 303/258 331/316 369/383 461/458 509/485; 12-bit tags
-// gain throughout (390/390 441/436 499/489 582/571 634/608).
-bool cuckoo_keys_together(const dtlg_filter* f) {
+// Cuckoo probes: keys tested one by one or together (contains_n), at 6 CTAs per
+// SM (variant 0) or 4 (1).  Tables that hit L1 on part of the loads only are
+// probed key by key at 4 CTAs: with more loads in flight the lines are gone
+// before they are used again.  us for 2^26 probes, 0 one by one / 0 together / 1
+// one by one / 1 together:
+//          16 KiB           200 KiB          320 KiB          512 KiB          64 MiB
+//   16/4   254/256/251/258  265/269/285/279  423/413/390/385  448/436/448/451  549/536/536/564
+//   16/1   251/253/243/247  261/261/274/264  407/421/398/381  438/430/455/463  544/530/537/564
+//   8/4    268/268/262/266  285/277/293/276  422/421/394/385  442/430/443/454  548/532/537/533
+//   4/4    341/342/342/346  363/353/363/354  445/440/397/419  470/457/476/500  578/560/568/601
+//   12/4   361/361/357/381  415/402/411/420  498/495/496/491  581/580/573/559  695/691/674/649
+//   32/2   219/222/218/230  250/252/256/261  396/414/400/374  441/433/449/441  551/536/537/560
+//   32/4   276/280/246/262  314/328/281/292  430/443/401/418  492/497/444/464  608/602/528/570
+// In two passes (beyond 64 MiB) more of the loads miss L2, and variant 0 with the
+// keys together is ahead: 16/4 at 146 MiB 853/841/979/888, 12/4 1057/1043/1122/1074;
+// buckets of 16 bytes from 120 MiB on (98 MiB 679/674/664/667, 146 MiB 834/800/942/831).
+struct CuckooForm {
+  int variant;
+  bool together;
+};
+CuckooForm cuckoo_form(const dtlg_filter* f) {
   const uint64_t kib = f->d.m_actual >> 13;
-  return f->d.t == 12 || kib > 512 || (kib <= 224 && f->d.t != 32);
+  const uint32_t t = f->d.t;
+  const bool two_pass = probe_passes(f) > 1;
+  if (t * f->d.b == 128) return two_pass && kib >= (120u << 10) ? CuckooForm{0, true} : CuckooForm{1, false};
+  if (two_pass) return {0, true};
+  if (kib >= 480) return {t == 12 ? 1 : 0, true};
+  if (kib >= 160 && kib < 230 && t != 12 && t != 32) return {0, true};
+  return {1, false};
 }
 
 // Variant of the bitmask kernel, 0 = 6 CTAs per SM (40 registers) or 1 = 4 (64
@@ -284,17 +315,12 @@ bool cuckoo_keys_together(const dtlg_filter* f) {
 //   u64 w=8 s=4          469/459 480/503 539/625     u32 w=16 z=4   375/374 378/394 502/521
 //   u32 w=16 s=1 k=4     444/442 450/432 489/498     u64 w=4 s=4    364/357 385/379 480/520
 //   u32 w=1 k=4          289/293 299/291 503/492     u64 w=16 k=16  717/611 723/659 784/761
+// (at 112 MiB u64 w=4 s=4 580/588, u32 w=8 s=8 477/485 at 96 MiB but 563/542 at 108)
 // (in one pass the 8-CTA, 32-register form was slower than 0 everywhere but for
 // u64 w=8 s=2 beyond 64 MiB, 723 at 96, and z=4 and s=4 at 80 to 96).  Bloom layouts whose
 // kernel 0 spills take kernel 1.
 int bits_variant_for(const dtlg_filter* f) {
-  if (f->ck) {
-    // two-pass tables miss L2 more (t=16 b=4, 142 MiB: 660 / 722; t=12 b=4, 106
-    // MiB 754 / 802); in one pass only 16-bit tags gain (510 / 532, 12-bit 640
-    // / 627, 8-bit 481 / 479, 32-bit 575 / 544), 12-bit ones up to 512 KiB (364
-    // / 384 at 16 KiB, 436 / 450 at 256)
-    return probe_passes(f) > 1 || f->d.t == 16 || (f->d.t == 12 && f->d.m_actual <= (512ull << 13)) ? 0 : 1;
-  }
+  if (f->ck) return cuckoo_form(f).variant;
   const uint64_t mib = f->d.m_actual >> 23;
   // classic Bloom, k = 4: 1 MiB 391 / 415, 64 MiB 427 / 485; k = 8 567 / 634,
   // 635 / 769; k = 2 340 / 332 at 8 MiB
@@ -302,7 +328,7 @@ int bits_variant_for(const dtlg_filter* f) {
   if (!f->bk || f->d.k > 8) return 1;
   const uint32_t block = f->d.w * f->d.word_bytes, s = f->d.s, w = f->d.w;
   const bool zoned = f->d.kind == Kind::kZoned, u32 = f->d.word_bytes == 4;
-  if (block == 32) return mib >= 68 && mib <= 116 ? 0 : 1;
+  if (block == 32) return mib >= 68 && mib <= (u32 ? 98 : 114) ? 0 : 1;
   if (block != 64) return 1;
   if (zoned) return (u32 && f->d.z == 2) || mib >= 60 ? 0 : 1;
   if (s >= w) return 0;
@@ -504,7 +530,7 @@ dtlg_status launch_probe(const dtlg_filter* f, const uint64_t* words, const uint
     // cuckoo buckets 75.6 -> 47.9, blocked cuckoo (128 MiB) 102.1 -> 98.9,
     // classic Bloom unchanged.
     a.l1na = (f->bk != nullptr && (f->d.m_actual / 8) > kL1NoAllocBytes) ? 1u : 0u;
-    a.together = cuckoo_keys_together(f) ? 1u : 0u;
+    a.together = f->ck != nullptr && cuckoo_form(f).together ? 1u : 0u;
     // match bitmask, in block-range passes over large filters (each pass
     // probes only the keys whose block lies in its range, so the concurrently
     // touched part of the filter stays within the GPU's address-translation reach)

@@ -107,15 +107,15 @@ template <class Ops, int MINB>
 __global__ void __launch_bounds__(256, MINB)
 probe_bits_kernel(const __grid_constant__ ProbeArgs a, uint32_t* __restrict__ bits, int or_into) {
   bits_loop(a, bits, or_into, [&](const uint32_t (&k)[4]) {
-    if constexpr (HasContainsN<Ops>::value) {
+    // two keys' loads in flight fit 40 registers, four spill
+    if constexpr (HasContainsN<Ops>::value && MINB >= 6) {
       if (a.together) {
-        // two keys' loads in flight fit 40 registers, four spill
-        if constexpr (MINB >= 6) {
-          const uint32_t lo[2] = {k[0], k[1]}, hi[2] = {k[2], k[3]};
-          return Ops::template contains_n<2>(a, lo) | Ops::template contains_n<2>(a, hi) << 2;
-        } else {
-          return Ops::template contains_n<4>(a, k);
-        }
+        const uint32_t lo[2] = {k[0], k[1]}, hi[2] = {k[2], k[3]};
+        return Ops::template contains_n<2>(a, lo) | Ops::template contains_n<2>(a, hi) << 2;
+      }
+    } else if constexpr (HasContainsN<Ops>::value) {
+      if constexpr (Ops::kTogetherAt4) {
+        if (a.together) return Ops::template contains_n<4>(a, k);
       }
     }
     uint32_t f = 0;
