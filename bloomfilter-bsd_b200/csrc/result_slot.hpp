@@ -40,13 +40,13 @@ class ResultSlots {
       for (int i = 0; i < kMax && !s; i++) {
         if (!made_[i]) {
           made_[i] = true;
+          slots_[i] = ResultSlot{};
           s = &slots_[i];
         }
       }
     }
     if (!s) return nullptr;
     RelaxedCapture relaxed;
-    *s = ResultSlot{};
     cudaError_t e = cudaMalloc(&s->dev, dev_bytes);
     if (e == cudaSuccess)
       e = cudaHostAlloc(reinterpret_cast<void**>(&s->host), 64, cudaHostAllocMapped | cudaHostAllocPortable);
