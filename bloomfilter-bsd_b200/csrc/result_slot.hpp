@@ -22,6 +22,7 @@ struct ResultSlot {
   unsigned long long* host_dev = nullptr;     // the same words, as the device sees them
   uint32_t ticket = 0;                        // of the slot's latest call
   bool fresh = true;                          // device scratch not zeroed yet
+  bool made = false;                          // in use or free, not dropped
 };
 
 // The slots of one device: a call takes one and gives it back, so threads and
@@ -37,11 +38,12 @@ class ResultSlots {
     {
       std::lock_guard<std::mutex> lk(mu_);
       if (n_free_ != 0) return free_[--n_free_];
-      for (int i = 0; i < kMax && !s; i++) {
-        if (!made_[i]) {
-          made_[i] = true;
-          slots_[i] = ResultSlot{};
-          s = &slots_[i];
+      for (ResultSlot& c : slots_) {
+        if (!c.made) {
+          c = ResultSlot{};
+          c.made = true;
+          s = &c;
+          break;
         }
       }
     }
@@ -72,7 +74,7 @@ class ResultSlots {
     if (s->dev) cudaFree(s->dev);
     if (s->host) cudaFreeHost(s->host);
     std::lock_guard<std::mutex> lk(mu_);
-    made_[s - slots_] = false;
+    s->made = false;
   }
 
  private:
@@ -86,7 +88,6 @@ class ResultSlots {
 
   std::mutex mu_;
   ResultSlot slots_[kMax];
-  bool made_[kMax] = {};
   ResultSlot* free_[kMax] = {};
   int n_free_ = 0;
 };
