@@ -583,7 +583,6 @@ dtlg_status launch_probe(const dtlg_filter* f, const uint64_t* words, const uint
   }
   const int cgrid = static_cast<int>(std::min<uint64_t>(tiles, static_cast<uint64_t>(ds->sms) * compact_occupancy()));
   switch (compact_rows(c.n_words)) {
-    case 1: compact_kernel<1><<<cgrid, kCompactThreads, 0, stream>>>(c); break;
     case 2: compact_kernel<2><<<cgrid, kCompactThreads, 0, stream>>>(c); break;
     case 4: compact_kernel<4><<<cgrid, kCompactThreads, 0, stream>>>(c); break;
     default: compact_kernel<8><<<cgrid, kCompactThreads, 0, stream>>>(c);

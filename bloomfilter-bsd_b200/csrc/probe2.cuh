@@ -6,7 +6,7 @@
 //    thing a warp ever waits for is its own filter loads.  probe_smem_kernel
 //    does the same against a copy of a small filter in shared memory.
 // 2. compact_kernel: turns the bitmask into the ascending position list.  A
-//    tile is 8192 to 65536 keys (256 to 2048 mask words, by the batch's size);
+//    tile is 16384 to 65536 keys (512 to 2048 mask words, by the batch's size);
 //    the tile offset comes from the tiles' status words, summed at once or by
 //    a decoupled look-back (bounded waits, as in probe.cuh).  It moves 1/8 byte per key in and 4 bytes per match out,
 //    staged per warp in shared memory so the stores are coalesced.
@@ -22,13 +22,19 @@
 namespace dtlg {
 
 constexpr int kCompactThreads = 256;
-// Tiles of 256 mask words (8192 keys) times `rows`: as few rows as give no more
-// than kCompactSumTiles tiles, so that batches of some million keys reach
-// every SM (5 M keys are 77 tiles of 65536) and the offsets are sums; then 8.
-constexpr uint32_t kCompactSumTiles = 1024;
+// Tiles of 256 mask words (8192 keys) times `rows`: 2 up to 2^21 keys, 4 up to
+// 2^25, 8 beyond, so that batches of some million keys reach many SMs without
+// more tickets and status words than a sparse mask is worth.  Between
+// kCompactSumMin and kCompactSumTiles tiles the offsets are sums, else a
+// look-back (few tiles publish before their successors look; beyond, the sums
+// read too many words).  us per probe (u32 w=1 k=4, 8 MiB) at 0 / 10 / 50 % hits,
+// tiles of 65536 keys throughout / of 8192 keys, as few as give 1024, by sums / so:
+//   2^20 19.2/21.0/29.9 20.4/20.0/20.7 16.9/16.8/18.8   2^21 23.5/25.9/35.8 25.0/25.3/26.3 21.6/22.3/25.1
+//   2^22 31.1/34.3/43.4 33.4/34.5/36.2 30.8/31.8/36.7   2^23 47.9/49.9/61.4 49.8/51.1/56.0 46.7/48.6/55.0
+//   2^24 87.0/90.1/100  86.8/88.4/94.2 83.3/85.6/93.2   2^25 154/159/175    153/157/169    152/157/169
+constexpr uint32_t kCompactSumMin = 512, kCompactSumTiles = 1024;
 __host__ __device__ constexpr uint32_t compact_rows(uint64_t n_words) {
-  return n_words <= 256ull * kCompactSumTiles ? 1 : n_words <= 512ull * kCompactSumTiles ? 2
-         : n_words <= 1024ull * kCompactSumTiles ? 4 : 8;
+  return n_words <= 1ull << 16 ? 2 : n_words <= 1ull << 20 ? 4 : 8;
 }
 constexpr uint32_t kMaxGatherCols = 4;
 
@@ -174,7 +180,7 @@ static __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const _
   ProbeArgs lb{};
   lb.status = a.status;
   lb.err = a.err;
-  const bool by_sum = a.n_tiles <= kCompactSumTiles;
+  const bool by_sum = a.n_tiles > kCompactSumMin && a.n_tiles <= kCompactSumTiles;
   for (;;) {
     if (threadIdx.x == 0) s_tile = atomicAdd(a.tile_ctr, 1u);
     __syncthreads();
@@ -265,6 +271,7 @@ static __global__ void __launch_bounds__(kCompactThreads) compact_kernel(const _
       __syncwarp();
       pos += tot;
     }
+    if (a.n_tiles <= gridDim.x) break;  // one tile per CTA
     __syncthreads();
   }
 }
