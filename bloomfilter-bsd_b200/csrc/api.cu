@@ -317,8 +317,8 @@ CuckooForm cuckoo_form(const dtlg_filter* f) {
 //   u32 w=1 k=4          289/293 299/291 503/492     u64 w=16 k=16  717/611 723/659 784/761
 // (at 112 MiB u64 w=4 s=4 580/588, u32 w=8 s=8 477/485 at 96 MiB but 563/542 at 108)
 // (in one pass the 8-CTA, 32-register form was slower than 0 everywhere but for
-// u64 w=8 s=2 beyond 64 MiB, 723 at 96, and z=4 and s=4 at 80 to 96).  Bloom layouts whose
-// kernel 0 spills take kernel 1.
+// u64 w=8 s=2 beyond 64 MiB, 723 at 96, and z=4 and s=4 at 80 to 96).  Bloom
+// layouts whose kernel 0 spills take kernel 1.
 int bits_variant_for(const dtlg_filter* f) {
   if (f->ck) return cuckoo_form(f).variant;
   const uint64_t mib = f->d.m_actual >> 23;
@@ -592,9 +592,10 @@ dtlg_status launch_probe(const dtlg_filter* f, const uint64_t* words, const uint
 }
 
 // Build plan of a blocked Bloom or blocked cuckoo filter (one block per key)
-// for n keys: 1 = one kernel of global atomics, 2 = keys grouped by L2-sized
-// block range first (the probe's partition).  Automatic: the partitioned
-// build for Bloom filters beyond 80 MiB and batches of >= 2^20 keys (u64 w=8
+// for n keys that are not built range by range (range_build): 1 = one kernel of
+// global atomics, 2 = keys grouped by L2-sized block range first (the probe's
+// partition).  Automatic: the partitioned build for Bloom filters beyond 80 MiB
+// and batches of >= 2^20 keys (u64 w=8
 // s=8 k=8, plan 1 -> plan 2: 512 MiB from 2^28 keys 10.55 -> 4.07 ms; 256 MiB
 // 4.23 -> 2.07 ms; 96 MiB (12 bits/key, MAGIC) 1.22 -> 1.09 ms; 64 MiB stays
 // with plan 1, 0.51 against 0.60 ms).  A blocked cuckoo key takes one or two
@@ -678,8 +679,9 @@ cudaError_t launch_range_build(const dtlg_filter* f, uint64_t* words, const uint
   ra.fill = reinterpret_cast<unsigned int*>(ws + bucket_bytes);
   ra.filter = words;
   // a range of the largest size has an SM to itself: while it is built, the
-  // one that the SM takes next comes into L2 (2^22 keys / 256 MiB 154 -> 132
-  // us; smaller ranges share the SM, and the hint only cost: 161 -> 181)
+  // one that the SM takes next comes into L2 (2^24 keys / 256 MiB 214 -> 206
+  // us, zoned u32 198 -> 188; full ranges gain nothing, 2^27 keys 1017 / 1014,
+  // u32 w=1 743 / 773; smaller ranges share the SM and take no hint)
   ra.prefetch = range_bytes == kBuildRangeBytes ? static_cast<uint32_t>(ds.sms) : 0u;
   set_range_layout(f->d.word_bytes, f->d.w,
                    make_schedule(f->d.word_bytes * 8, f->d.w, f->d.s, f->d.z, f->d.k, true), &ra);

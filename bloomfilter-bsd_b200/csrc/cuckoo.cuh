@@ -412,7 +412,7 @@ __device__ __forceinline__ void cuckoo_insert_key(const CuckooBuildArgs& a, uint
 // thread with their loads and first swaps in flight together was slower (129
 // against 103 us: the buckets are chosen on older counts, so more keys kick).
 // t=16 b=4, 3 000 001 keys at load 0.9: 199 us with unpack, pack and random
-// kicks, 103 us so; 2^26 keys at load 0.95 7.4 -> 2.8 ms.
+// kicks, about 100 us so; 2^26 keys at load 0.95 7.4 -> 2.8 ms.
 template <class Cfg>
 __global__ void __launch_bounds__(256) cuckoo_insert_kernel(const __grid_constant__ CuckooBuildArgs a) {
   using S = typename std::conditional<Cfg::kWordBucket, WordBuckets<Cfg>, SlotBuckets<Cfg>>::type;

@@ -137,7 +137,8 @@ dtlg_status dtlg_batch_insert_host(const dtlg_filter* f, uint64_t* words, const 
   if (failed_out) *failed_out = 0;
   if (n == 0) return DTLG_OK;
   if (dtlg_kind(f) == 2) {
-    // cuckoo: one insert over all keys (each call unpacks and repacks the table)
+    // cuckoo: one insert over all keys (each call ends with a synchronization, and
+    // unpacks and repacks tables whose buckets are no 16-, 32- or 64-bit word)
     if (n > 0xFFFFFFFFull) return DTLG_ERR_SIZE;
     uint32_t* d = nullptr;
     PIPE_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&d), n * 4 + 16, stream));

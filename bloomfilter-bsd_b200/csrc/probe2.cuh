@@ -8,8 +8,9 @@
 // 2. compact_kernel: turns the bitmask into the ascending position list.  A
 //    tile is 16384 to 65536 keys (512 to 2048 mask words, by the batch's size);
 //    the tile offset comes from the tiles' status words, summed at once or by
-//    a decoupled look-back (bounded waits, as in probe.cuh).  It moves 1/8 byte per key in and 4 bytes per match out,
-//    staged per warp in shared memory so the stores are coalesced.
+//    a decoupled look-back (bounded waits, as in probe.cuh).  It moves 1/8 byte
+//    per key in and 4 bytes per match out, staged per warp in shared memory so
+//    the stores are coalesced.
 // The extra traffic against the fused kernel is the bitmask, 2/8 byte per key.
 #pragma once
 

@@ -140,7 +140,8 @@ class filter_base:  # noqa: N801 (reference name)
 
     def set_build_options(self, mode=0):
         """Bloom build plan: 0 automatic, 1 one kernel of global atomic ORs,
-        2 keys grouped by L2-sized block range first (same words)."""
+        2 keys grouped by L2-sized block range first (same words; inserts into
+        the same words may run at the same time under every plan)."""
         check(lib().dtlg_set_build_options(self._h, int(mode)), "set_build_options")
 
     def build_plan(self, key_cnt):

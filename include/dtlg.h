@@ -190,15 +190,19 @@ dtlg_status dtlg_batch_contains_gather(const dtlg_filter* f, const uint64_t* fil
  * blocked_bloomfilter_tune.hpp:21-56.) */
 dtlg_status dtlg_set_probe_options(dtlg_filter* f, int mode, int variant);
 /* Build plan of a blocked Bloom or blocked cuckoo filter (no counterpart in
- * the reference, whose batch_insert is one loop): 0 = automatic (large batches
- * range by range in shared memory; else 2 for Bloom filters beyond 80 MiB and
- * batches of >= 2^20 keys, else 1), 1 = one kernel of
+ * the reference, whose batch_insert is one loop): 0 = automatic (for Bloom
+ * filters, batches of >= 2^22 keys into filters of enough 8 to 128 KiB ranges
+ * are built range by range in shared memory, from 4.3 to 5 bytes per key of
+ * workspace; else 2 beyond 80 MiB and 2^20 keys, else 1), 1 = one kernel of
  * global atomics, 2 = keys first grouped by ~8 MiB block range (the
- * partitioned probe's partition, ~8.3 bytes per key of workspace from the
- * library's stream-ordered pool; without room there, plan 1), then inserted
- * range by range so the atomics hit L2.  Bloom filter
- * words are the same under every plan; blocked cuckoo builds are randomised
- * under both (as the reference's); other filter kinds ignore it. */
+ * partitioned probe's partition, ~8.3 bytes per key of workspace), then
+ * inserted range by range so the atomics hit L2.  The workspaces come from the
+ * library's stream-ordered pool, which keeps its memory for later calls;
+ * without room there, and for the range-by-range build under stream capture,
+ * the next plan in line is taken.  Bloom filter words are the same under every
+ * plan, and every plan ORs them atomically: Bloom inserts into the same words
+ * may run at the same time.  Blocked cuckoo builds are randomised under both
+ * (as the reference's); other filter kinds ignore it. */
 dtlg_status dtlg_set_build_options(dtlg_filter* f, int mode);
 /* The plan that one batch_insert of key_cnt keys takes with the current
  * options: 1 and 2 as above, 3 = range by range in shared memory; 0 for no
@@ -270,7 +274,9 @@ dtlg_status dtlg_batch_contains_noalloc(const dtlg_filter* f, const uint64_t* fi
  * allocates and copies; the buffers named by the items must stay valid and
  * unchanged); dtlg_batch_run then builds and probes all filters in ONE
  * persistent kernel (optionally replayed as a CUDA graph).  Results are those
- * of the per-filter calls: each item's filter words after inserting its build
+ * of the per-filter calls (items must not share filter words, and nothing else
+ * may insert into them during a run: the kernel reads a range's words, ORs and
+ * stores them): each item's filter words after inserting its build
  * keys, and its probe keys' ascending match positions + count (DEVICE).
  * Bloom filters of the compiled menu (u64 w=8 s=8 k=8; zoned u64 w=8 and u32
  * w=16 with z=2/4, k=8; u32 w=1 k=4/8) run inside the persistent kernel;
