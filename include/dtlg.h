@@ -204,8 +204,8 @@ dtlg_status dtlg_set_probe_options(dtlg_filter* f, int mode, int variant);
  * may run at the same time.  Blocked cuckoo builds are randomised under both
  * (as the reference's); other filter kinds ignore it. */
 dtlg_status dtlg_set_build_options(dtlg_filter* f, int mode);
-/* The plan that one batch_insert of key_cnt keys takes with the current
- * options: 1 and 2 as above, 3 = range by range in shared memory; 0 for no
+/* The plan that one batch_insert of key_cnt keys (16-byte aligned) takes with
+ * the current options: 1 and 2 as above, 3 = range by range in shared memory; 0 for no
  * filter or no keys.  (A batch whose workspace finds no room, or that is
  * captured into a graph, takes 1 or 2 instead of 3.) */
 int dtlg_build_plan(const dtlg_filter* f, uint32_t key_cnt);
